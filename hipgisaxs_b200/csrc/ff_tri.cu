@@ -18,6 +18,8 @@
 //  * ff_tri_f64_kernel     — the plain FP64 form: one thread per q-point, triangles staged
 //                            through shared memory, reference arithmetic.  Parity reference
 //                            on the device and the denominator of the FP32 speed-up.
+//  * ff_tri_mma_kernel     — (ff_tri_mma.cu) FP32C on detector-row grids with the sums on the tensor
+//                            cores; the automatic choice nearly everywhere (rows_mma_pays).
 //  * ff_tri_rows_kernel    — FP32, for q-grids laid out by detector rows (QGrid layout: qz
 //                            depends on the row only).  The rotation is folded into the
 //                            triangles (q'.c = q.(R^T c)), the phase splits into an in-plane
@@ -39,29 +41,15 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <mutex>
 
+#include "ff_tri.cuh"
+#include "ff_tri_mma.cuh"
 #include "hgx_internal.cuh"
 #include "ptx.cuh"
 
 namespace hgx {
 
-constexpr int TILE = TRI_TILE;              // triangles per shared-memory tile (512)
-constexpr int TILE_FLOATS = TILE * 6;       // float4 A[TILE] (dx,nx,dy,ny) + float2 B[TILE] (dz,nz)
-constexpr uint32_t TILE_BYTES = TILE_FLOATS * 4;
 constexpr int TILE_X2_FLOATS = TILE * 10;   // float4 A2[2*TILE] ((dx,dx,dy,dy),(nx,nx,ny,ny)) + float2 B[TILE]
 constexpr uint32_t TILE_X2_BYTES = TILE_X2_FLOATS * 4;
-constexpr double TWO_PI = 6.283185307179586476925286766559;
-constexpr double INV_TWO_PI = 0.15915494309189533576888376337251;
-constexpr float TWO_PI_F = 6.28318530717958648f;
-constexpr float INV_TWO_PI_F = 0.159154943091895336f;
-// In-plane phases of a tile with |q_par| * (largest offset) above 8 pi radians get the
-// explicit reduction to [-1/2, 1/2] turn before the SFU; below it they go straight in (the SFU
-// reduces its argument itself; its error grows with |x| by the rounding of x / 2 pi, about
-// 2^-24 |x|, 1.5e-6 rad at 8 pi).
-constexpr float WIDE_PHASE2 = 631.65468f;   // (8 pi)^2
-
-struct Rot9 {
-  double r[9];
-};
 
 // ------------------------------------------------------------- triangle prep ----
 // Morton order: bounding box of the centroids (per-block partials, then one block), 30-bit
@@ -165,13 +153,16 @@ __global__ void tri_key_kernel(const double* __restrict__ sd, int ntri, const do
 // FP32x2 pairs; the packed layout in turns), its anchor (c0x/2pi, c0y/2pi, c0z, max |d_par|)
 // and, when perm is not NULL, the triangle index of each slot (-1 for padding).  The anchor's
 // sums run in a fixed order (deterministic).  Padding slots are zero (they contribute nothing).
+// xy, info (scalar layout, may be NULL): the extra arrays of the tensor-core kernel (MmaTiles).
 template <bool X2>
 __global__ void __launch_bounds__(TILE) tri_tile_kernel(const double* __restrict__ sd, int ntri, Rot9 R,
                                                         const int* __restrict__ order,
                                                         float* __restrict__ tiles,
                                                         double4* __restrict__ anchors,
-                                                        int* __restrict__ perm) {
+                                                        int* __restrict__ perm, float* __restrict__ xy,
+                                                        float4* __restrict__ info) {
   __shared__ double s_red[TILE / 32][4];
+  __shared__ float s_info[TILE / 32][3];
   __shared__ double s_c0[3];
   __shared__ double s_rmax[TILE / 32];
   const int tile = blockIdx.x, j = threadIdx.x;
@@ -235,62 +226,41 @@ __global__ void __launch_bounds__(TILE) tri_tile_kernel(const double* __restrict
     float2* B = reinterpret_cast<float2*>(tiles + (size_t)tile * TILE_FLOATS + 4 * TILE);
     A[j] = make_float4(dx, nx, dy, ny);
     B[j] = make_float2(dz, nz);
-  }
-}
-
-// ------------------------------------------------------------------ helpers ----
-__device__ __forceinline__ void two_sum_fold(float& sum, float& part, float& comp) {
-  float s = sum + part;
-  float bp = s - sum;
-  float err = (sum - (s - bp)) + (part - bp);
-  sum = s;
-  comp += err;
-  part = 0.f;
-}
-
-// |R (qx, qy, qz)|^2 with complex qz, as RotMatrix_t::rotate + cuCnorm3 evaluate it.
-__device__ __forceinline__ double rotated_q2(const Rot9& R, double qx, double qy, double2 qz) {
-  double q2 = 0.0;
+    if (xy) {
+      float* v = xy + (size_t)tile * MMA_XY + (j >> 1) * 4 + (j & 1);
+      v[0] = dx;
+      v[2] = dy;
+      // the tile's largest |n~| component (infinite when one is not finite: the form factor is
+      // then NaN) and its range of dz
+      float m = fmaxf(fmaxf(fabsf(nx), fabsf(ny)), fabsf(nz)), lo = dz, hi = dz;
+      if (!isfinite(nx + ny + nz)) m = INFINITY;
 #pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    double re = R.r[3 * j] * qx + R.r[3 * j + 1] * qy + R.r[3 * j + 2] * qz.x;
-    double im = R.r[3 * j + 2] * qz.y;
-    q2 += re * re + im * im;
+      for (int o = 16; o > 0; o >>= 1) {
+        m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
+        lo = fminf(lo, __shfl_down_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_down_sync(0xffffffffu, hi, o));
+      }
+      if ((j & 31) == 0) {
+        s_info[j >> 5][0] = m;
+        s_info[j >> 5][1] = lo;
+        s_info[j >> 5][2] = hi;
+      }
+      __syncthreads();
+      if (j == 0) {
+        for (int w = 1; w < TILE / 32; ++w) {
+          m = fmaxf(m, s_info[w][0]);
+          lo = fminf(lo, s_info[w][1]);
+          hi = fmaxf(hi, s_info[w][2]);
+        }
+        float rm = (float)s_rmax[0];
+        for (int w = 1; w < TILE / 32; ++w) rm = fmaxf(rm, (float)s_rmax[w]);
+        float* e = xy + (size_t)tile * MMA_XY + 2 * TILE;
+        e[0] = rm;
+        e[1] = e[2] = e[3] = 0.f;
+        info[tile] = make_float4(m, lo, hi, 0.f);
+      }
+    }
   }
-  return q2;
-}
-
-template <typename OUT>
-__device__ __forceinline__ void store_ff(OUT* out, long idx, double re, double im);
-template <>
-__device__ __forceinline__ void store_ff<float2>(float2* out, long idx, double re, double im) {
-  out[idx] = make_float2((float)re, (float)im);
-}
-template <>
-__device__ __forceinline__ void store_ff<double2>(double2* out, long idx, double re, double im) {
-  out[idx] = make_double2(re, im);
-}
-
-// The anchor phasor e^{2 pi i u} of an FP64 phase u in turns, reduced exactly in FP64.
-__device__ __forceinline__ float2 anchor_phasor(double u) {
-  u -= rint(u);
-  float s, c;
-  sincospif((float)(2.0 * u), &s, &c);
-  return make_float2(c, s);
-}
-
-// (re, im) <- (re, im) * (c + i s)
-__device__ __forceinline__ void rotate_pair(float& re, float& im, float2 a) {
-  const float r = re * a.x - im * a.y;
-  im = re * a.y + im * a.x;
-  re = r;
-}
-
-// Rounds x to the nearest integer (ties to even) with two FP32 adds — valid for
-// |x| < 2^22 — so the reduction stays on the FMA pipe instead of the conversion unit.
-__device__ __forceinline__ float round_nearest(float x) {
-  const float magic = 12582912.0f;  // 1.5 * 2^23
-  return (x + magic) - magic;
 }
 
 // ------------------------------------------------------------- row kernel ----
@@ -306,30 +276,6 @@ struct RowArgs {
   void* out;
   unsigned* err;
 };
-
-// Row factor of one (row, triangle) for a real block pair (qz, -qz), cz in turns (FP64):
-// Z = e^{i 2pi qz cz} = (x, y), D = qz n~z; returns (x, y, D*y, D*x).
-__device__ __forceinline__ float4 paired_factor(double q, double cz, float nz) {
-  double u = q * cz;
-  u -= rint(u);
-  float s, c;
-  sincospif((float)(2.0 * u), &s, &c);
-  float D = (float)(q * (double)nz);
-  return make_float4(c, s, D * s, D * c);
-}
-
-// Row factor for a general complex block, cz in turns: Z = e^{i 2pi qz cz}, D = qz n~z;
-// returns (Z, D Z).
-__device__ __forceinline__ float4 complex_factor(double2 q, double cz, float nz) {
-  double u = q.x * cz;
-  u -= rint(u);
-  double amp = exp(-TWO_PI * q.y * cz);
-  double s, c;
-  sincospi(2.0 * u, &s, &c);
-  double zr = amp * c, zi = amp * s;
-  double dr = q.x * (double)nz, di = q.y * (double)nz;
-  return make_float4((float)zr, (float)zi, (float)(dr * zr - di * zi), (float)(dr * zi + di * zr));
-}
 
 // One tile's partial sums of the row kernel (see ff_tri_rows_kernel).  WIDE: the in-plane
 // phases get the explicit reduction to [-1/2, 1/2] turn before the SFU.
@@ -982,6 +928,8 @@ struct TilePrep {
   float* tiles = nullptr;
   double4* anchors = nullptr;
   int* perm = nullptr;
+  float* xy = nullptr;
+  float4* info = nullptr;
   unsigned* keys[2] = {nullptr, nullptr};
   int* idx[2] = {nullptr, nullptr};
   double* bbox = nullptr;
@@ -1006,9 +954,9 @@ static int prepare_tiles(hgx_ctx c, const double* sd, int ntri, const Rot9& R, b
                                              (unsigned*)nullptr, (const int*)nullptr, (int*)nullptr,
                                              ntri, 0, 30, st));
   }
-  size_t off[9];
+  size_t off[11];
   size_t total = 0;
-  const size_t sizes[9] = {tile_bytes,
+  const size_t sizes[11] = {tile_bytes,
                            sizeof(double4) * (size_t)ntiles,
                            sizeof(int) * (size_t)ntiles * TILE,
                            sort ? sizeof(unsigned) * (size_t)ntri : 0,
@@ -1016,8 +964,10 @@ static int prepare_tiles(hgx_ctx c, const double* sd, int ntri, const Rot9& R, b
                            sort ? sizeof(int) * (size_t)ntri : 0,
                            sort ? sizeof(int) * (size_t)ntri : 0,
                            sort ? sizeof(double) * 6 * (size_t)nparts : 0,
-                           sort_bytes};
-  for (int i = 0; i < 9; ++i) {
+                           sort_bytes,
+                           x2 ? 0 : sizeof(float) * MMA_XY * (size_t)ntiles,
+                           x2 ? 0 : sizeof(float4) * (size_t)ntiles};
+  for (int i = 0; i < 11; ++i) {
     off[i] = total;
     total += align256(sizes[i]);
   }
@@ -1027,6 +977,10 @@ static int prepare_tiles(hgx_ctx c, const double* sd, int ntri, const Rot9& R, b
   t.tiles = reinterpret_cast<float*>(base + off[0]);
   t.anchors = reinterpret_cast<double4*>(base + off[1]);
   t.perm = reinterpret_cast<int*>(base + off[2]);
+  if (!x2) {
+    t.xy = reinterpret_cast<float*>(base + off[9]);
+    t.info = reinterpret_cast<float4*>(base + off[10]);
+  }
   const int* order = nullptr;
   if (sort) {
     t.keys[0] = reinterpret_cast<unsigned*>(base + off[3]);
@@ -1046,13 +1000,26 @@ static int prepare_tiles(hgx_ctx c, const double* sd, int ntri, const Rot9& R, b
     order = t.idx[1];
   }
   if (x2)
-    tri_tile_kernel<true><<<ntiles, TILE, 0, st>>>(sd, ntri, R, order, t.tiles, t.anchors, t.perm);
+    tri_tile_kernel<true><<<ntiles, TILE, 0, st>>>(sd, ntri, R, order, t.tiles, t.anchors, t.perm,
+                                                   nullptr, nullptr);
   else
-    tri_tile_kernel<false><<<ntiles, TILE, 0, st>>>(sd, ntri, R, order, t.tiles, t.anchors, t.perm);
+    tri_tile_kernel<false><<<ntiles, TILE, 0, st>>>(sd, ntri, R, order, t.tiles, t.anchors, t.perm, t.xy,
+                                                    t.info);
   HGX_CUDA(cudaGetLastError());
   c->tiles = TileView{t.tiles, t.anchors, t.perm, ntiles, ntri};
   *out = t;
   return HGX_OK;
+}
+
+// The tensor-core row kernel takes row grids of any width: its unit is 128 columns, but even a
+// narrow grid is faster there (16 x 16 x 1,280 triangles: 0.059 against 0.122 ms; 48 x 256: 0.090
+// against 0.123; 130 x 512 x 4,800: 0.52 against 0.90; complex blocks 1.4 to 4.4 times faster at
+// every size tried).  The FP32 row kernel keeps one corner: real blocks, at most 64 columns and
+// rows that fill its two CTAs per SM at one pixel per thread (64 x 1024 x 4,800: 0.515 against
+// 0.560 ms; at 300 rows 0.320 against 0.245, from 8 CTAs of 4 rows per 4 SMs on 3.4 against 1.07).
+static bool rows_mma_pays(hgx_ctx c, hgx_qgrid g) {
+  const int ctas = (g->nrow + 3) / 4;
+  return !(g->mode == 1 && g->ncol <= 64 && 4 * ctas >= 7 * c->sm_count && ctas < 2 * c->sm_count);
 }
 
 int ff_triangles_device(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, const double* rot9,
@@ -1067,6 +1034,14 @@ int ff_triangles_device(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, cons
     else ff_tri_f64_kernel<128, double2><<<grid, 128, 0, st>>>(a);
     HGX_CUDA(cudaGetLastError());
     return HGX_OK;
+  }
+  if (want_p == 0 && g->tuned_p == 0 && g->mode != 0 && rows_mma_pays(c, g)) {
+    if (row_shape(g->nrow, g->ncol, c->sm_count, 4).grid.y > 65535u)
+      return fail(HGX_ERR_INVALID_ARG, "hgx_ff_triangles: too many detector rows for one launch");
+    TilePrep t;
+    HGX_TRY(prepare_tiles(c, sd, ntri, R, false, &t));
+    const int s = ff_rows_mma(c, g, MmaTiles{t.tiles, t.anchors, t.xy, t.info, c->tiles.ntiles, ntri}, R, out, ff_type);
+    if (s != HGX_ERR_NO_MEMORY) return s;  // without room for the row factors: the row kernels below
   }
   if (want_p == 0) want_p = g->tuned_p;  // the autotuner's choice for this grid, if any
   if (want_p != 0 && want_p != 1 && want_p != 2 && want_p != 4 && want_p != -2 && want_p != -4 &&
@@ -1392,7 +1367,7 @@ extern "C" int hgx_ff_triangles_noalloc(const double* shape_def, int ntri, int n
   // tiles in the caller's triangle order (no sort, which would need more scratch), each with
   // its FP64 anchor
   tri_tile_kernel<false><<<ntiles, TILE, 0, st>>>(shape_def, ntri, R, nullptr, slot.tiles,
-                                                 slot.anchors, nullptr);
+                                                 slot.anchors, nullptr, nullptr, nullptr);
   HGX_CUDA(cudaGetLastError());
   PointArgs a{slot.tiles, slot.anchors, ntiles, qx, qy, reinterpret_cast<const double2*>(qz), nqy,
               nqz, R, ff, slot.err};

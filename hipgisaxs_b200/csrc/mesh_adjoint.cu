@@ -532,10 +532,10 @@ int hgx_mesh_chi2_grad_ex(hgx_ctx c, hgx_qgrid g, int nv, const double* verts, i
   mesh_to_shape_kernel<<<(nf + 127) / 128, 128, 0, st>>>((const double*)dv, nv, (const int*)df, nf,
                                                          (double*)sd.p, c->d_err);
   HGX_TRY(F.reserve((f64 ? sizeof(double2) : sizeof(float2)) * 4 * n));
-  // FP32C: the scalar row kernel (4 pixels/thread), whose triangle tiles the backward pass
+  // FP32C: the row kernels in the scalar tile layout, whose triangle tiles the backward pass
   // reads; FP64: the plain FP64 kernel
   HGX_TRY(ff_triangles_device(c, g, (const double*)sd.p, nf, R, precision, F.p,
-                              f64 ? HGX_C128 : HGX_C64, 4));
+                              f64 ? HGX_C128 : HGX_C64, g->tuned_p ? 4 : 0));
   // 3. intensity, chi^2, seeds
   const int sblocks = (int)((n + 255) / 256);
   HGX_TRY(seeds.reserve((f64 ? sizeof(double4) : sizeof(float4)) * 2 * n));

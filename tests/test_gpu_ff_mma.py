@@ -1,0 +1,75 @@
+"""The tensor-core row kernel of the FP32C triangle form factor (the automatic choice on row grids).
+
+Bound: the project's FP32C tolerance, 1e-5 norm-wise against the FP64 oracle.  Each term's error
+is at most that of the SFU sine and cosine and of the 22- and 24-bit digits, about 1e-6 of the
+tile's largest triangle, so sums that do not cancel below a tenth of their terms stay inside.
+"""
+import numpy as np
+import pytest
+
+import hipgisaxs_b200 as hg
+from hipgisaxs_b200 import meshes
+
+pytestmark = pytest.mark.gpu
+TOL32 = 1e-5
+
+
+def cloud(rng, T, scale=6.0):
+    sd = np.zeros((T, 8))
+    sd[:, 0] = rng.uniform(0.2, 3.0, T)
+    n = rng.normal(size=(T, 3))
+    sd[:, 1:4] = n / np.linalg.norm(n, axis=1)[:, None]
+    sd[:, 4:7] = rng.normal(scale=scale, size=(T, 3))
+    return sd
+
+
+def detector(po, ncol, nrow, kind):
+    """(qx, qy, qz) of a detector grid: four real blocks, four complex ones, or one complex."""
+    G = po.Grid(ncol, nrow, -1.9, 0.0, 2.0, 3.0, 0.2, 10.0, (6e-6, 8e-8) if kind != "real" else (0.0, 0.0))
+    return G.qx, G.qy, G.qz_ext[:ncol * nrow].copy() if kind == "one" else G.qz_ext
+
+
+@pytest.mark.parametrize("kind", ["real", "complex", "one"])
+@pytest.mark.parametrize("ncol,nrow,ntri", [
+    (2, 3, 1), (17, 5, 31), (127, 2, 32), (128, 2, 33), (129, 2, 511), (64, 3, 512), (257, 2, 513),
+    (40, 3, 1500),   # tiles split over CTAs
+    (130, 9, 4700),  # ten tiles: stages and accumulators reused
+])
+def test_edges_of_tiles_chunks_and_columns(ctx, po, kind, ncol, nrow, ntri):
+    rng = np.random.default_rng(1000 * ncol + ntri)
+    sd = cloud(rng, ntri)
+    R = po.rot_mul(po.rot_axis(2, 0.2), po.rot_axis(1, 0.1))
+    qx, qy, qz = detector(po, ncol, nrow, kind)
+    g = hg.QGrid.from_arrays(ctx, qx, qy, qz, ncol)
+    assert g.mode == (1 if kind == "real" else 2)
+    ref = po.ff_approx_triangle(sd, qx, qy, qz, R)
+    for out_type in ("c128", "c64"):
+        f = hg.ff_triangles(ctx, g, sd, R, "f32c", out_type=out_type)
+        ok = np.isfinite(ref)  # a q-point at q = 0 is 0 / 0 in both
+        assert np.array_equal(ok, np.isfinite(f)) and po.rel_err(f[ok], ref[ok]) < TOL32
+
+
+def test_wide_phases(ctx, po):
+    """One tile spread over 2 um: its in-plane phases take the explicit reduction."""
+    sd = cloud(np.random.default_rng(5), 300, scale=400.0)
+    qx, qy, qz = detector(po, 130, 4, "real")
+    g = hg.QGrid.from_arrays(ctx, qx, qy, qz, 130)
+    assert po.rel_err(hg.ff_triangles(ctx, g, sd, None, "f32c"), po.ff_approx_triangle(sd, qx, qy, qz)) < TOL32
+
+
+def test_slabs_of_row_factors(ctx, po):
+    """More row factors than are held at a time: several slabs of rows, against the FP64 kernel."""
+    V, F = meshes.star_mesh(15.0, 125, 81)
+    sd = meshes.shape_def_from_mesh(V, F)
+    g = hg.QGrid.create(ctx, 16, 1500, -1.9, 0.0, 2.0, 3.0, 0.0035, 50.677)
+    f64 = hg.ff_triangles(ctx, g, sd, None, "f64")
+    assert po.rel_err(hg.ff_triangles(ctx, g, sd, None, "f32c"), f64) < TOL32
+
+
+@pytest.mark.parametrize("col,value", [(0, np.nan), (0, np.inf), (2, np.nan), (5, np.nan), (6, np.inf)])
+def test_a_triangle_that_is_not_finite_is_not_hidden(ctx, po, col, value):
+    sd = cloud(np.random.default_rng(6), 600)
+    sd[70, col] = value
+    qx, qy, qz = detector(po, 33, 3, "real")
+    g = hg.QGrid.from_arrays(ctx, qx, qy, qz, 33)
+    assert not np.isfinite(hg.ff_triangles(ctx, g, sd, None, "f32c")).any()

@@ -42,7 +42,7 @@
 #include <mutex>
 
 #include "ff_tri.cuh"
-#include "ff_tri_mma.cuh"
+#include "ff_tri_rows.cuh"
 #include "hgx_internal.cuh"
 #include "ptx.cuh"
 
@@ -1028,6 +1028,10 @@ int ff_triangles_device(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, cons
   Rot9 R = make_rot(rot9);
   const bool c64 = ff_type == HGX_C64;
   if (precision == HGX_F64) {
+    if (g->mode != 0) {
+      const int s = ff_rows_f64(c, g, sd, ntri, R, out, ff_type);
+      if (s != HGX_ERR_NO_MEMORY) return s;
+    }
     F64Args a{sd, ntri, g->qx, g->qy, g->qz, g->nqy, g->nqz, R, out};
     dim3 grid((g->nqz + 127) / 128);
     if (c64) ff_tri_f64_kernel<128, float2><<<grid, 128, 0, st>>>(a);

@@ -41,7 +41,7 @@
 
 #include <algorithm>
 
-#include "ff_tri_mma.cuh"
+#include "ff_tri_rows.cuh"
 #include "ptx.cuh"
 #include "tc05.cuh"
 

@@ -1,4 +1,5 @@
-// The tensor-core row kernel of the FP32C triangle form factor (ff_tri_mma.cu).
+// The row-grid kernels of the triangle form factor: FP32C on the tensor cores (ff_tri_mma.cu) and
+// FP64 (ff_tri_f64.cu).
 #pragma once
 
 #include "ff_tri.cuh"
@@ -21,5 +22,8 @@ struct MmaTiles {
 
 // Enqueues the form factor of a row grid (g->mode 1 or 2).
 int ff_rows_mma(hgx_ctx c, hgx_qgrid g, const MmaTiles& t, const Rot9& R, void* out, int ff_type);
+
+// The same in FP64.  HGX_ERR_NO_MEMORY: nothing was enqueued, the plain kernel takes the call.
+int ff_rows_f64(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, const Rot9& R, void* out, int ff_type);
 
 }  // namespace hgx

@@ -123,15 +123,16 @@ static int fill_dist(Dist& d, int n, const double* v, const double* w, const cha
     d.v[i] = v[i];
     d.w[i] = w ? w[i] : 1.0;
   }
-  // evenly stepped samples (the FP32C cylinder sums their height exponentials in closed form)
+  // evenly stepped samples (the cylinder sums their height exponentials in closed form: FP32C
+  // within 1e-12, FP64 within the rounding of the steps)
   d.prog = 0;
   if (n >= 3) {
     const double step = (v[n - 1] - v[0]) / (n - 1);
     double big = 0.0;
     for (int i = 0; i < n; ++i) big = std::max(big, std::fabs(v[i]));
-    bool prog = step != 0.0;
-    for (int i = 0; i < n && prog; ++i) prog = std::fabs(v[i] - (v[0] + i * step)) <= 1e-12 * big;
-    d.prog = prog ? 1 : 0;
+    double off = 0.0;
+    for (int i = 0; i < n; ++i) off = std::max(off, std::fabs(v[i] - (v[0] + i * step)));
+    d.prog = step != 0.0 && off <= 1e-12 * big ? (off <= 1e-14 * big ? 2 : 1) : 0;
   }
   return HGX_OK;
 }

@@ -98,6 +98,7 @@ struct HigWork {
   int arena_cur = 0;
   size_t arena_off = 0;  // nonzero between a simulation's first copy and its end
   DevBuf fc, ff, eff, sf, I, img, shapes, elems, gt, er, sc, obj, saxs_qz, ratios;
+  DevBuf gpart;  // sums of the FP64 grain kernel's splits
   DevBuf ftab;  // the fused grain kernel's tables of one structure, as one block
   // the objective's gradient: the tables' changes, d(distance)/d(image), d(image)/dx
   DevBuf tshapes, telems, tgt, ter, tsc, lam, dimg;

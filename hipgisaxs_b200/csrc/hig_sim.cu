@@ -52,6 +52,7 @@
 
 #include "ana_sf.cuh"
 #include "ana_sf_f32.cuh"
+#include "ana_sf_real.cuh"
 #include "ana_sf_tangent.cuh"
 #include "hgx_internal.cuh"
 #include "hig_config.hpp"
@@ -182,6 +183,7 @@ struct FusedArgs {
   double* out;             // N intensities, accumulated
   // a population launch (grid y = candidate): per-candidate strides of shapes, elems and
   // scales (records), grains and elem_rot (doubles) and out (doubles); 0 otherwise
+  double* part = nullptr;  // grain_dwba_real_kernel with grid z > 1: the splits' sums
   long ps_shape = 0, ps_elem = 0, ps_grain = 0, ps_er = 0, ps_scale = 0, ps_out = 0;
 };
 
@@ -341,9 +343,154 @@ __global__ void __launch_bounds__(128) grain_dwba_f32c_kernel(FusedArgs a) {
   if (live && k == 0) out[i] = acc;
 }
 
-// true when the FP32C grain kernel has a body for this shape
+// The fused grain loop in FP64 for grids with real qz and unit cells of one shape among cylinder,
+// sphere and box: one thread per pixel holds the four DWBA blocks, so that what does not depend on
+// the block is made once.  For a grain turned about z ("flat": qz stays out of the rotated in-plane
+// q) that is the a- and b-axis lattice factors (one division for both) and the in-plane form
+// factor; the centre's in-plane phase, common to the four terms, drops out of |sum|^2.  When two
+// successive grains also leave the elements' form factors unchanged (cylinders and spheres
+// turned about their axis, without an in-plane offset), fc_k ff_k are kept: such an ensemble costs
+// little more than its lattice factors, about 260 FP64 operations per (pixel, grain) with the
+// c axis, where grain_dwba_kernel's complex powers, logarithms and exponentials took 6,400.
+// Bound by the FP64 pipe.  Grains of a launch are split over grid z where a small image leaves SMs
+// idle; the splits' sums are added in order by grain_sum_kernel.
+template <int SHAPE>
+__device__ __forceinline__ void grain_terms(const FusedArgs& a, const AnaShape* shapes, const FusedElem* elems,
+                                            const double* er, double qx, double qy, const double (&qz)[4],
+                                            const zd (&fc)[4], zd (&f)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) f[k] = zd(0, 0);
+  for (int e = 0; e < a.nelem; ++e, er += 9) {
+    const AnaShape& sh = shapes[e];
+    const double* loc = elems[e].loc;
+    const zd dn2(elems[e].dre, elems[e].dim);
+    const bool flat = er[2] == 0.0 && er[5] == 0.0, moved = loc[0] != 0.0 || loc[1] != 0.0 || loc[2] != 0.0;
+    const double p0 = er[0] * qx + er[1] * qy, p1 = er[3] * qx + er[4] * qy, p2 = er[6] * qx + er[7] * qy;
+    double in = 0.0;
+    if (SHAPE != SH_SPHERE && flat) in = ff_inplane_real<SHAPE>(sh, p0, p1);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const double m0 = p0 + er[2] * qz[k], m1 = p1 + er[5] * qz[k], m2 = p2 + er[8] * qz[k];
+      zd v;
+      if (SHAPE == SH_SPHERE) v = sphere_real(sh.d[0], m0, m1, m2);
+      else v = ff_axial_real<SHAPE>(sh, m2) * (flat ? in : ff_inplane_real<SHAPE>(sh, m0, m1));
+      if (moved) v = v * expi_real(m0 * loc[0] + m1 * loc[1] + m2 * loc[2]);
+      f[k] += dn2 * v;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) f[k] = fc[k] * f[k];
+}
+
+// The elements' form factors are those of the grain before (see grain_dwba_real_kernel).
+template <int SHAPE>
+__device__ __forceinline__ bool same_elements(const FusedArgs& a, const FusedElem* elems, const double* er) {
+  if (SHAPE == SH_BOX) return false;
+  for (int e = 0; e < a.nelem; ++e, er += 9) {
+    const double* b = er - 9 * (long)a.nelem;
+    if (er[2] != 0.0 || er[5] != 0.0 || er[6] != 0.0 || er[7] != 0.0 || b[2] != 0.0 || b[5] != 0.0 ||
+        b[6] != 0.0 || b[7] != 0.0 || er[8] != b[8] || elems[e].loc[0] != 0.0 || elems[e].loc[1] != 0.0)
+      return false;
+  }
+  return true;
+}
+
+template <int SHAPE>
+__global__ void __launch_bounds__(128, 4) grain_dwba_real_kernel(FusedArgs a) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  const double qx = a.qx[i], qy = a.qy[i];
+  double qz[4];
+  zd fc[4], f[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    qz[k] = a.qz[k * a.n + i].x;
+    fc[k] = zd(a.fc[k * a.n + i]);
+  }
+  const long cy = blockIdx.y;  // the candidate of a population launch
+  const AnaShape* shapes = a.shapes + cy * a.ps_shape;
+  const FusedElem* elems = a.elems + cy * a.ps_elem;
+  const double* grains = a.grains + cy * a.ps_grain;
+  const double* elem_rot = a.elem_rot + cy * a.ps_er;
+  const ScaleEntry* scales = a.scales + cy * a.ps_scale;
+  const int ng = a.g1 - a.g0;
+  const int ga = a.g0 + (int)((long)blockIdx.z * ng / gridDim.z), gb = a.g0 + (int)((long)(blockIdx.z + 1) * ng / gridDim.z);
+  double* out = gridDim.z > 1 ? a.part + (long)blockIdx.z * a.n : a.out + cy * a.ps_out;
+  double acc = gridDim.z > 1 ? 0.0 : out[i];
+  for (int g = ga; g < gb; ++g) {
+    const double* gp = grains + 12 * (long)g;
+    const double* er = elem_rot + 9 * (long)g * a.nelem;
+    if (g == ga || !same_elements<SHAPE>(a, elems, er)) grain_terms<SHAPE>(a, shapes, elems, er, qx, qy, qz, fc, f);
+    const bool flat = gp[2] == 0.0 && gp[5] == 0.0;
+    const double p0 = gp[0] * qx + gp[1] * qy, p1 = gp[3] * qx + gp[4] * qy, p2 = gp[6] * qx + gp[7] * qy;
+    const double cx = gp[9], cyy = gp[10], cz = gp[11];
+    const bool centred = cx == 0.0 && cyy == 0.0 && cz == 0.0;
+    const ScaleEntry* sp = scales + (long)g * a.nscale;
+    for (int si = 0; si < a.nscale; ++si) {
+      const ScaleEntry& L = sp[si];
+      zd sum(0, 0);
+      double ab = 1.0;
+      if (a.sfbuf) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sum += f[k] * zd(a.sfbuf[k * a.n + i]);
+      } else if (flat && L.la[2] == 0.0) {
+        const Ratio ra = dirichlet_real((p0 * L.la[0] + p1 * L.la[1]) * INV_2PI_R, L.rep[0]);
+        const Ratio rb = dirichlet_real((p0 * L.lb[0] + p1 * L.lb[1] + L.lb[2] * L.lb[2]) * INV_2PI_R, L.rep[1]);
+        ab = (ra.num * rb.num) / (ra.den * rb.den);
+        const double tc = p0 * L.lc[0] + p1 * L.lc[1] + p2 * L.lc[2], zc = gp[8] * L.lc[2];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          zd v = f[k];
+          if (L.rep[2] != 1.0) {
+            const Ratio rc = dirichlet_real((tc + zc * qz[k]) * INV_2PI_R, L.rep[2]);
+            v = v * (rc.num / rc.den);
+          }
+          if (cz != 0.0) v = v * expi_real(gp[8] * qz[k] * cz);  // the rest of the phase is common
+          sum += v;
+        }
+      } else {
+#pragma unroll 1
+        for (int k = 0; k < 4; ++k) {
+          const double q = k == 0 ? qz[0] : k == 1 ? qz[1] : k == 2 ? qz[2] : qz[3];
+          const zd fk = k == 0 ? f[0] : k == 1 ? f[1] : k == 2 ? f[2] : f[3];
+          const double m0 = p0 + gp[2] * q, m1 = p1 + gp[5] * q, m2 = p2 + gp[8] * q;
+          const double ub = (m0 * L.lb[0] + m1 * L.lb[1] + L.lb[2] * L.lb[2]) * INV_2PI_R;
+          const Ratio ra = dirichlet_real((m0 * L.la[0] + m1 * L.la[1] + m2 * L.la[2]) * INV_2PI_R, L.rep[0]);
+          const Ratio rb = dirichlet_real(ub, L.rep[1]);
+          const Ratio rc = dirichlet_real((m0 * L.lc[0] + m1 * L.lc[1] + m2 * L.lc[2]) * INV_2PI_R, L.rep[2]);
+          zd v = fk * (ra.num * rb.num * rc.num / (ra.den * rb.den * rc.den));
+          if (L.rep[1] != round_fp64(L.rep[1])) v = v * dirichlet_b_phase(ub, L.rep[1]);
+          if (!centred) v = v * expi_real(m0 * cx + m1 * cyy + m2 * cz);
+          sum += v;
+        }
+      }
+      const double w = L.w * ab;
+      acc += w * w * (sum.x * sum.x + sum.y * sum.y);
+    }
+  }
+  out[i] = acc;
+}
+
+// out += the splits' sums, in order.
+__global__ void grain_sum_kernel(const double* __restrict__ part, int splits, long n, double* __restrict__ out) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double v = out[i];
+  for (int s = 0; s < splits; ++s) v += part[(long)s * n + i];
+  out[i] = v;
+}
+
+// true when the real-qz grain kernels (FP32C and FP64) have a body for this shape
 static bool grain_f32c_shape(int shape) {
   return shape == SH_CYLINDER || shape == SH_SPHERE || shape == SH_BOX;
+}
+
+static void launch_grain_real(int shape, dim3 grid, cudaStream_t st, const FusedArgs& a) {
+  switch (shape) {
+    case SH_CYLINDER: grain_dwba_real_kernel<SH_CYLINDER><<<grid, 128, 0, st>>>(a); break;
+    case SH_SPHERE: grain_dwba_real_kernel<SH_SPHERE><<<grid, 128, 0, st>>>(a); break;
+    default: grain_dwba_real_kernel<SH_BOX><<<grid, 128, 0, st>>>(a); break;
+  }
 }
 
 static void launch_grain_f32c(int shape, unsigned blocks, cudaStream_t st, const FusedArgs& a) {
@@ -471,6 +618,7 @@ static void launch_grain_tangent(int shape, unsigned blocks, cudaStream_t st, co
 }
 
 constexpr int FUSED_GRAINS_PER_LAUNCH = 64;  // keeps each launch to tens of milliseconds
+constexpr int REAL_GRAINS_PER_LAUNCH = 2048;
 
 template <int PAIRED>
 void launch_grain_kernel(int shape, unsigned blocks, cudaStream_t st, const FusedArgs& a) {
@@ -929,6 +1077,23 @@ static int fused_structure(hgx_ctx c, hgx_qgrid g, HigWork& w, const hig::Struct
     if (shapes[e].shape != one) one = 0;
   // FP32C: grids with real qz blocks (paired rows) and one shape with an FP32C body
   const bool f32c = precision == HGX_F32C && g->mode == 1 && grain_f32c_shape(one);
+  if (!f32c && g->mode == 1 && grain_f32c_shape(one)) {
+    const unsigned blocks1 = (unsigned)((a.n + 127) / 128);
+    // four CTAs of 128 threads run per SM; grains are split where the pixels do not fill them
+    const int splits = (int)std::max<long>(1, std::min<long>({4L * c->sm_count / blocks1, (long)ngr / 4, 32}));
+    if (splits > 1) {
+      HGX_TRY(w.gpart.reserve(sizeof(double) * a.n * splits));
+      a.part = (double*)w.gpart.p;
+    }
+    for (int g0 = 0; g0 < ngr; g0 += REAL_GRAINS_PER_LAUNCH) {
+      a.g0 = g0;
+      a.g1 = std::min(ngr, g0 + REAL_GRAINS_PER_LAUNCH);
+      launch_grain_real(one, dim3(blocks1, 1, splits), st, a);
+      if (splits > 1) grain_sum_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a.part, splits, a.n, a.out);
+      HGX_CUDA(cudaGetLastError());
+    }
+    return HGX_OK;
+  }
   for (int g0 = 0; g0 < ngr; g0 += FUSED_GRAINS_PER_LAUNCH) {
     a.g0 = g0;
     a.g1 = g0 + FUSED_GRAINS_PER_LAUNCH < ngr ? g0 + FUSED_GRAINS_PER_LAUNCH : ngr;
@@ -1536,6 +1701,7 @@ namespace {
 struct PopStruct {
   int ngr = 0, nscale = 0, nelem = 0, shape = 0;
   bool liquid = false, f32c = false;
+  bool real = false;  // FP64 on real qz: grain_dwba_real_kernel
   // byte offsets in the staging block of each table's region; a region holds the table of every
   // candidate in turn (candidate i at i x the table's size)
   size_t o_shapes = 0, o_elems = 0, o_gt = 0, o_er = 0, o_sc = 0;
@@ -1651,7 +1817,9 @@ int pop_enqueue(hgx_hig_pop_s& P, cudaStream_t st) {
     for (int g0 = 0; g0 < ps.ngr; g0 += chunk) {
       a.g0 = g0;
       a.g1 = std::min(ps.ngr, g0 + chunk);
-      if (ps.f32c) {
+      if (ps.real) {
+        launch_grain_real(ps.shape, dim3((unsigned)((n + 127) / 128), (unsigned)P.npop), st, a);
+      } else if (ps.f32c) {
         switch (ps.shape) {
           case SH_CYLINDER: grain_dwba_f32c_kernel<SH_CYLINDER><<<grid, 128, 0, st>>>(a); break;
           case SH_SPHERE: grain_dwba_f32c_kernel<SH_SPHERE><<<grid, 128, 0, st>>>(a); break;
@@ -1793,6 +1961,7 @@ int hgx_hig_population_create(hgx_ctx c, hgx_hig h, int npop, const double* ref,
     ps.shape = t.shape;
     ps.liquid = t.liquid;
     ps.f32c = precision == HGX_F32C && g->mode == 1 && grain_f32c_shape(t.shape);
+    ps.real = !ps.f32c && g->mode == 1 && grain_f32c_shape(t.shape);
     ps.n_gt = t.f.gt.size();
     ps.n_er = t.f.er.size();
     ps.n_sc = t.plan.size();
@@ -1878,7 +2047,7 @@ int hgx_hig_population_eval(hgx_hig_pop p, const double* X, int nx, double* dist
   const int chunk = pop_chunk(p->npop);
   for (int k = 0; k < p->nstruct; ++k) {
     const PopStruct& ps = p->st[k];
-    if (ps.f32c) continue;
+    if (ps.f32c || ps.real) continue;
     for (int g0 = 0; g0 < ps.ngr; g0 += chunk) v.push_back(pop_paired(all, k, g0, std::min(ps.ngr, g0 + chunk)));
   }
   if (p->exec && v != p->variants) {  // another kernel variant: record the graph again

@@ -1,6 +1,6 @@
-// FP32 phase helpers of the FP32C kernels that keep work off the SFU/conversion (XU) pipe:
+// Phase helpers.  FP32, for the FP32C kernels, that keep work off the SFU/conversion (XU) pipe:
 // rounding to an integer by adding and subtracting a power-of-two constant (FP64 or FP32 add
-// pipe), and sin/cos of pi x by polynomials on the FMA pipe.
+// pipe), and sin/cos of pi x by polynomials on the FMA pipe.  FP64: sin/cos of phases in turns.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -46,10 +46,9 @@ __device__ __forceinline__ void sincospi_f32(float x, float* s, float* c) {
 // of degree 6 in r^2 (Chebyshev fits over the interval; both within 1.4e-16 of the value).  18 FP64
 // operations.  Valid for |u| < 2^50; NaN and infinite u give NaN.
 __device__ __forceinline__ void sincos_turns(double u, double* s, double* c) {
-  const double magic = 6755399441055744.0;  // 1.5 2^52
-  const double t = fma(u, 4.0, magic);
+  const double t = fma(u, 4.0, RND52);
   const int k = __double2loint(t);
-  const double r = fma(t - magic, -0.25, u), z = r * r;
+  const double r = fma(t - RND52, -0.25, u), z = r * r;
   double p = 3.780830078125, q = -1.698876953125;
   p = fma(p, z, -15.093802528381348);
   q = fma(q, z, 7.9031996917724605);
@@ -69,6 +68,28 @@ __device__ __forceinline__ void sincos_turns(double u, double* s, double* c) {
   const double a = odd ? q : p, b = odd ? p : q;
   *s = __hiloint2double(__double2hiint(a) ^ ((k & 2) << 30), __double2loint(a));
   *c = __hiloint2double(__double2hiint(b) ^ (((k + 1) & 2) << 30), __double2loint(b));
+}
+
+// sin of 2 pi r for |r| <= 1/4 (a polynomial of degree 8 in r^2 times r, a Chebyshev fit; within
+// 2.6e-16 of the value, relative near 0), and of 2 pi u for any |u| < 2^50, reduced exactly by the
+// nearest half turn.  10 and 13 FP64 operations.
+__device__ __forceinline__ double sin_quarter_turn(double r) {
+  const double z = r * r;
+  double p = 0.100869140625;
+  p = fma(p, z, -0.7177266693115234);
+  p = fma(p, z, 3.8199273419380186);
+  p = fma(p, z, -15.094641633983702);
+  p = fma(p, z, 42.058693924097824);
+  p = fma(p, z, -76.70585975280203);
+  p = fma(p, z, 81.60524927607344);
+  p = fma(p, z, -41.341702240399755);
+  p = fma(p, z, 6.283185307179586);
+  return p * r;
+}
+__device__ __forceinline__ double sin_turns(double u) {
+  const double t = fma(u, 2.0, RND52);
+  const double s = sin_quarter_turn(fma(t - RND52, -0.5, u));
+  return __hiloint2double(__double2hiint(s) ^ (__double2loint(t) << 31), __double2loint(s));
 }
 
 }  // namespace hgx

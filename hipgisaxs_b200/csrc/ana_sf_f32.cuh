@@ -1,8 +1,9 @@
-// FP32-compensated bodies of the fused grain kernel (hig_sim.cu) for a real rotated q (grids
-// whose DWBA qz blocks are real: a vacuum particle layer): the cylinder, sphere and box form
-// factors and the lattice structure factor of the reference's formulas, with every phase
-// formed and range-reduced in FP64 and only the transcendental of the reduced argument (and
-// the sums) in FP32.  Grids with complex qz keep the FP64 bodies of ana_sf.cuh.
+// FP32-compensated bodies for a real rotated q (grids whose DWBA qz blocks are real: a vacuum
+// particle layer) of the form- and structure-factor kernels and, in part, of the fused grain
+// kernel: the cylinder, sphere and box form factors and the lattice structure factor of the
+// reference's formulas, with every phase formed and range-reduced in FP64 and only the
+// transcendental of the reduced argument (and the sums) in FP32.  Grids with complex qz keep the
+// FP64 bodies of ana_sf.cuh.
 //
 // Lattice structure factor (src/sf/sf.cpp:164-246): for a real angle theta the reference's
 // principal-branch expression
@@ -165,57 +166,6 @@ __device__ __forceinline__ cf ff_analytic_f32c(const AnaShape& a, const double* 
   return out;
 }
 
-// The quad of four lanes (one per DWBA block) of the fused grain kernel: the sum of v over the
-// quad, the same bits in every lane (an xor butterfly of commutative adds).
-__device__ __forceinline__ float quad_sum(float v) {
-  v += __shfl_xor_sync(0xffffffffu, v, 1);
-  v += __shfl_xor_sync(0xffffffffu, v, 2);
-  return v;
-}
-
-// ff_analytic_f32c for a quad whose rotated in-plane q (m[0], m[1]) is the same in its four
-// lanes (the element's rotation keeps qz out of them): what depends on the in-plane q only - the
-// cylinder's radial sum, the box's x and y sums - is split among the lanes (lane k takes the
-// samples k, k + 4, ...) and summed by quad_sum; the qz parts stay per lane.  Every lane of the
-// warp calls it (shuffles); the sphere, whose |q| involves qz, keeps ff_analytic_f32c.
-template <int SHAPE>
-__device__ __forceinline__ cf ff_analytic_f32c_quad(const AnaShape& a, const double* m, const double* tv, int k) {
-  const Dist& X = a.d[0];
-  const Dist& Y = a.d[1];
-  const Dist& Z = a.d[2];
-  if (SHAPE == SH_CYLINDER) {
-    const double qpar = sqrt(m[0] * m[0] + m[1] * m[1]);
-    float fr = 0.f;
-    for (int i = k; i < X.n; i += 4) {
-      const double r = X.v[i], x = qpar * r;
-      if (x * x > CUTINY_REF) fr += (float)(2. * PI_REF * r * r) * (j1f((float)x) / (float)x);
-    }
-    fr = quad_sum(fr);
-    const cf gh = cyl_height_sum_f32(Z, m[2]);
-    return with_phase_f(cscale(gh, fr), m, tv);
-  } else if (SHAPE == SH_BOX) {
-    float sx = 0.f, sy = 0.f;
-    for (int i = k; i < X.n; i += 4) {
-      const double x = m[0] * 0.5 * X.v[i];
-      sx += sinc_from(x, expi_f(x).y) * (float)(X.v[i] * X.w[i]);
-    }
-    for (int i = k; i < Y.n; i += 4) {
-      const double x = m[1] * 0.5 * Y.v[i];
-      sy += sinc_from(x, expi_f(x).y) * (float)(Y.v[i] * Y.w[i]);
-    }
-    sx = quad_sum(sx);
-    sy = quad_sum(sy);
-    cf sz{0.f, 0.f};
-    for (int i = 0; i < Z.n; ++i) {
-      const double x = m[2] * 0.5 * Z.v[i];
-      const cf e = expi_f(x);
-      sz = cadd(sz, cscale(e, sinc_from(x, e.y) * (float)(Z.v[i] * Z.w[i])));
-    }
-    return with_phase_f(cscale(sz, sx * sy), m, tv);
-  }
-  return ff_analytic_f32c<SHAPE>(a, m, tv);
-}
-
 // sin(N theta_r / 2) / sin(theta_r / 2) on the principal angle theta_r of e^{i theta}
 __device__ __forceinline__ float dirichlet_principal(double theta, double N) {
   if (N == 1.0) return 1.f;
@@ -254,24 +204,6 @@ __device__ __forceinline__ cf sf_lattice_f32c(const SfLat& L, const double* m) {
   const float sc = dirichlet_principal(tc, L.rep[2]);
   const cf t3 = expi_f(m[0] * L.center[0] + m[1] * L.center[1] + m[2] * L.center[2]);
   return cmul(t3, cscale(sb, sa * sc));
-}
-
-// sf_lattice_f32c for a quad whose rotated in-plane q is the same in its four lanes, with an
-// in-plane a vector and an integer b repetition: the a- and b-axis factors do not depend on
-// the block, so the even lanes evaluate the a factor and the odd lanes the b factor (the same
-// code on other arguments) and a shuffle exchanges them; the c factor and the centre phase
-// stay per lane.  Every lane of the warp calls it.
-__device__ __forceinline__ cf sf_lattice_f32c_paired(const SfLat& L, const double* m, int k) {
-  const bool odd = (k & 1) != 0;
-  const double th = odd ? m[0] * L.lb[0] + m[1] * L.lb[1] + L.lb[2] * L.lb[2]
-                        : m[0] * L.la[0] + m[1] * L.la[1] + m[2] * L.la[2];
-  const float own = dirichlet_principal(th, odd ? L.rep[1] : L.rep[0]);
-  const float other = __shfl_xor_sync(0xffffffffu, own, 1);
-  const float sa = odd ? other : own, sb = odd ? own : other;
-  const double tc = m[0] * L.lc[0] + m[1] * L.lc[1] + m[2] * L.lc[2];
-  const float sc = dirichlet_principal(tc, L.rep[2]);
-  const cf t3 = expi_f(m[0] * L.center[0] + m[1] * L.center[1] + m[2] * L.center[2]);
-  return cscale(t3, sb * sa * sc);
 }
 
 }  // namespace hgx

@@ -267,119 +267,52 @@ __global__ void __launch_bounds__(128, (SHAPE == SH_PYRAMID || SHAPE == 0) ? 3 :
   if (live && k == 0) out[i] = acc;
 }
 
-// The fused grain loop in FP32C for grids with real qz and unit cells of one shape among
-// cylinder, sphere and box: the same quad layout and order of sums as grain_dwba_kernel, the
-// form and structure factors from ana_sf_f32.cuh (FP64 phases, FP32 transcendentals and
-// sums), the DWBA terms in FP32 and the intensity accumulated in FP64.
-template <int SHAPE>
-__global__ void __launch_bounds__(128) grain_dwba_f32c_kernel(FusedArgs a) {
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long i = t >> 2;
-  const int k = (int)(t & 3);
-  const bool live = i < a.n;  // every lane takes part in the shuffles
-  const long ii = live ? i : 0;
-  const double qx = a.qx[ii], qy = a.qy[ii];
-  const double qz = a.qz[k * a.n + ii].x;
-  const double2 fcd = a.fc[k * a.n + ii];
-  const cf fc{(float)fcd.x, (float)fcd.y};
-  const int base = (threadIdx.x & 31) & ~3;
-  const long cy = blockIdx.y;  // the candidate of a population launch
-  const AnaShape* shapes = a.shapes + cy * a.ps_shape;
-  const FusedElem* elems = a.elems + cy * a.ps_elem;
-  const double* grains = a.grains + cy * a.ps_grain;
-  const double* elem_rot = a.elem_rot + cy * a.ps_er;
-  const ScaleEntry* scales = a.scales + cy * a.ps_scale;
-  double* out = a.out + cy * a.ps_out;
-  double acc = (live && k == 0) ? out[i] : 0.0;
-  for (int g = a.g0; g < a.g1; ++g) {
-    const double* gp = grains + 12 * (long)g;
-    cf ff{0.f, 0.f};
-    for (int e = 0; e < a.nelem; ++e) {
-      const double* er = elem_rot + 9 * ((long)g * a.nelem + e);
-      double m[3];
-#pragma unroll
-      for (int j = 0; j < 3; ++j) m[j] = er[3 * j] * qx + er[3 * j + 1] * qy + er[3 * j + 2] * qz;
-      // the same grain and element in every lane of the warp: the test is warp-uniform; the
-      // split pays when the in-plane sums have four samples or more
-      const cf eff = (er[2] == 0.0 && er[5] == 0.0 && shapes[e].d[0].n >= 4)
-                         ? ff_analytic_f32c_quad<SHAPE>(shapes[e], m, elems[e].loc, k)
-                         : ff_analytic_f32c<SHAPE>(shapes[e], m, elems[e].loc);
-      ff = cadd(ff, cmul(cf{(float)elems[e].dre, (float)elems[e].dim}, eff));
-    }
-    double mr[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) mr[j] = gp[3 * j] * qx + gp[3 * j + 1] * qy + gp[3 * j + 2] * qz;
-    const ScaleEntry* sp = scales + (long)g * a.nscale;
-    const bool flat = gp[2] == 0.0 && gp[5] == 0.0;  // the grain rotation keeps qz out of mr[0], mr[1]
-    for (int si = 0; si < a.nscale; ++si) {
-      cf sfv;
-      if (a.sfbuf) {
-        const double2 v = a.sfbuf[k * a.n + ii];
-        sfv = cf{(float)v.x, (float)v.y};
-      } else {
-        SfLat L;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          L.la[d] = sp[si].la[d];
-          L.lb[d] = sp[si].lb[d];
-          L.lc[d] = sp[si].lc[d];
-          L.rep[d] = sp[si].rep[d];
-          L.center[d] = gp[9 + d];
-        }
-        // warp-uniform: the same grain and sample in every lane
-        sfv = (flat && L.la[2] == 0.0 && L.rep[1] == round_fp64(L.rep[1])) ? sf_lattice_f32c_paired(L, mr, k)
-                                                                           : sf_lattice_f32c(L, mr);
-      }
-      const cf term = cmul(cmul(fc, sfv), ff);
-      cf sum{0.f, 0.f};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        sum = cadd(sum, cf{__shfl_sync(0xffffffffu, term.x, base + j),
-                           __shfl_sync(0xffffffffu, term.y, base + j)});
-      const float w = (float)sp[si].w;
-      acc += (double)(w * w * (sum.x * sum.x + sum.y * sum.y));
-    }
-  }
-  if (live && k == 0) out[i] = acc;
-}
-
-// The fused grain loop in FP64 for grids with real qz and unit cells of one shape among cylinder,
-// sphere and box: one thread per pixel holds the four DWBA blocks, so that what does not depend on
-// the block is made once.  For a grain turned about z ("flat": qz stays out of the rotated in-plane
-// q) that is the a- and b-axis lattice factors (one division for both) and the in-plane form
-// factor; the centre's in-plane phase, common to the four terms, drops out of |sum|^2.  When two
-// successive grains also leave the elements' form factors unchanged (cylinders and spheres
-// turned about their axis, without an in-plane offset), fc_k ff_k are kept: such an ensemble costs
-// little more than its lattice factors, about 260 FP64 operations per (pixel, grain) with the
-// c axis, where grain_dwba_kernel's complex powers, logarithms and exponentials took 6,400.
-// Bound by the FP64 pipe.  Grains of a launch are split over grid z where a small image leaves SMs
-// idle; the splits' sums are added in order by grain_sum_kernel.
-template <int SHAPE>
+// The fused grain loop for grids with real qz and unit cells of one shape among cylinder, sphere
+// and box, T = double (FP64) or float (FP32C: FP64 phases, FP32 transcendentals and sums, the
+// intensity accumulated in FP64).  One thread per pixel holds the four DWBA blocks, so that what
+// does not depend on the block is made once: for a grain turned about z ("flat": qz stays out of
+// the rotated in-plane q) that is the a- and b-axis lattice factors and the in-plane form factor;
+// the centre's in-plane phase, common to the four terms, drops out of |sum|^2.  When two
+// successive grains also leave the elements' form factors unchanged (cylinders and spheres turned
+// about their axis, without an in-plane offset), fc_k ff_k are kept: such an ensemble costs little
+// more than its lattice factors.  The rotated lattice vectors of a batch of grains are made once
+// per CTA, in turns (shared memory), so that an angle is two or three multiply-adds.
+//
+// Bound by the FP64 pipe (T = double: 230 FP64 operations per (pixel, grain) with a c axis, where
+// grain_dwba_kernel's complex powers, logarithms and exponentials take 6,400) or by issue (float).
+// 600 x 300 pixels x 625 grains, 100 x 10 x 2 cells: FP64 2.16 ms (63.5 on grain_dwba_kernel), FP32C
+// 1.3 ms (10.0 on four threads per pixel); four CTAs of 128 registers per SM (3: 3.2 ms, 6: 2.6 at
+// an earlier step of 2.5).  Grains of a launch are split over grid z where a small image leaves
+// SMs idle; grain_sum_kernel adds the splits' sums in order.
+template <typename T, int SHAPE>
 __device__ __forceinline__ void grain_terms(const FusedArgs& a, const AnaShape* shapes, const FusedElem* elems,
-                                            const double* er, double qx, double qy, const double (&qz)[4],
-                                            const zd (&fc)[4], zd (&f)[4]) {
+                                            const double* er, double qx, double qy, const double (&qz)[4], long i,
+                                            cx<T> (&f)[4]) {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) f[k] = zd(0, 0);
+  for (int k = 0; k < 4; ++k) f[k] = cx<T>{0, 0};
   for (int e = 0; e < a.nelem; ++e, er += 9) {
     const AnaShape& sh = shapes[e];
     const double* loc = elems[e].loc;
-    const zd dn2(elems[e].dre, elems[e].dim);
+    const cx<T> dn2{(T)elems[e].dre, (T)elems[e].dim};
     const bool flat = er[2] == 0.0 && er[5] == 0.0, moved = loc[0] != 0.0 || loc[1] != 0.0 || loc[2] != 0.0;
     const double p0 = er[0] * qx + er[1] * qy, p1 = er[3] * qx + er[4] * qy, p2 = er[6] * qx + er[7] * qy;
-    double in = 0.0;
-    if (SHAPE != SH_SPHERE && flat) in = ff_inplane_real<SHAPE>(sh, p0, p1);
+    T in = 0;
+    if (SHAPE != SH_SPHERE && flat) in = ff_inplane_real<T, SHAPE>(sh, p0, p1);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const double m0 = p0 + er[2] * qz[k], m1 = p1 + er[5] * qz[k], m2 = p2 + er[8] * qz[k];
-      zd v;
-      if (SHAPE == SH_SPHERE) v = sphere_real(sh.d[0], m0, m1, m2);
-      else v = ff_axial_real<SHAPE>(sh, m2) * (flat ? in : ff_inplane_real<SHAPE>(sh, m0, m1));
-      if (moved) v = v * expi_real(m0 * loc[0] + m1 * loc[1] + m2 * loc[2]);
-      f[k] += dn2 * v;
+      cx<T> v;
+      if (SHAPE == SH_SPHERE) v = sphere_real<T>(sh.d[0], m0, m1, m2);
+      else v = (flat ? in : ff_inplane_real<T, SHAPE>(sh, m0, m1)) * ff_axial_real<T, SHAPE>(sh, m2);
+      if (moved) v = v * expi_real<T>(m0 * loc[0] + m1 * loc[1] + m2 * loc[2]);
+      f[k] = f[k] + dn2 * v;
     }
   }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) f[k] = fc[k] * f[k];
+  for (int k = 0; k < 4; ++k) {
+    const double2 c = a.fc[k * a.n + i];
+    f[k] = cx<T>{(T)c.x, (T)c.y} * f[k];
+  }
 }
 
 // The elements' form factors are those of the grain before (see grain_dwba_real_kernel).
@@ -395,18 +328,24 @@ __device__ __forceinline__ bool same_elements(const FusedArgs& a, const FusedEle
   return true;
 }
 
-template <int SHAPE>
+// One structure-factor evaluation of a grain: the angles of the axes and of the centre's phase are
+// q . vector, in turns (b: plus b0, the reference's lb[2] lb[2] term).
+struct GrainAngles {
+  double a[3], b[3], c[3], d[3], b0, rep[3], w;
+  int flat, keep;  // a and b without qz; the elements' form factors are those of the grain before
+};
+constexpr int GRAIN_BATCH = 32;
+
+template <typename T, int SHAPE>
 __global__ void __launch_bounds__(128, 4) grain_dwba_real_kernel(FusedArgs a) {
+  __shared__ GrainAngles s_g[GRAIN_BATCH];
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  const double qx = a.qx[i], qy = a.qy[i];
+  const bool live = i < a.n;
+  const long ii = live ? i : 0;
+  const double qx = a.qx[ii], qy = a.qy[ii];
   double qz[4];
-  zd fc[4], f[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    qz[k] = a.qz[k * a.n + i].x;
-    fc[k] = zd(a.fc[k * a.n + i]);
-  }
+  for (int k = 0; k < 4; ++k) qz[k] = a.qz[k * a.n + ii].x;
   const long cy = blockIdx.y;  // the candidate of a population launch
   const AnaShape* shapes = a.shapes + cy * a.ps_shape;
   const FusedElem* elems = a.elems + cy * a.ps_elem;
@@ -416,59 +355,86 @@ __global__ void __launch_bounds__(128, 4) grain_dwba_real_kernel(FusedArgs a) {
   const int ng = a.g1 - a.g0;
   const int ga = a.g0 + (int)((long)blockIdx.z * ng / gridDim.z), gb = a.g0 + (int)((long)(blockIdx.z + 1) * ng / gridDim.z);
   double* out = gridDim.z > 1 ? a.part + (long)blockIdx.z * a.n : a.out + cy * a.ps_out;
-  double acc = gridDim.z > 1 ? 0.0 : out[i];
-  for (int g = ga; g < gb; ++g) {
-    const double* gp = grains + 12 * (long)g;
-    const double* er = elem_rot + 9 * (long)g * a.nelem;
-    if (g == ga || !same_elements<SHAPE>(a, elems, er)) grain_terms<SHAPE>(a, shapes, elems, er, qx, qy, qz, fc, f);
-    const bool flat = gp[2] == 0.0 && gp[5] == 0.0;
-    const double p0 = gp[0] * qx + gp[1] * qy, p1 = gp[3] * qx + gp[4] * qy, p2 = gp[6] * qx + gp[7] * qy;
-    const double cx = gp[9], cyy = gp[10], cz = gp[11];
-    const bool centred = cx == 0.0 && cyy == 0.0 && cz == 0.0;
-    const ScaleEntry* sp = scales + (long)g * a.nscale;
-    for (int si = 0; si < a.nscale; ++si) {
-      const ScaleEntry& L = sp[si];
-      zd sum(0, 0);
-      double ab = 1.0;
+  double acc = gridDim.z > 1 ? 0.0 : out[ii];
+  cx<T> f[4];
+  for (long e0 = (long)ga * a.nscale; e0 < (long)gb * a.nscale; e0 += GRAIN_BATCH) {
+    const int ne = (int)min((long)GRAIN_BATCH, (long)gb * a.nscale - e0);
+    __syncthreads();
+    if (threadIdx.x < ne) {
+      const long e = e0 + threadIdx.x;
+      const int g = (int)(e / a.nscale);
+      const double* R = grains + 12 * (long)g;
+      const ScaleEntry L = scales[e];
+      GrainAngles& G = s_g[threadIdx.x];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {  // q'.v = q.(R^T v); the b axis without its z component
+        G.a[j] = (R[j] * L.la[0] + R[3 + j] * L.la[1] + R[6 + j] * L.la[2]) * INV_2PI_R;
+        G.b[j] = (R[j] * L.lb[0] + R[3 + j] * L.lb[1]) * INV_2PI_R;
+        G.c[j] = (R[j] * L.lc[0] + R[3 + j] * L.lc[1] + R[6 + j] * L.lc[2]) * INV_2PI_R;
+        G.d[j] = (R[j] * R[9] + R[3 + j] * R[10] + R[6 + j] * R[11]) * INV_2PI_R;
+        G.rep[j] = L.rep[j];
+      }
+      G.b0 = L.lb[2] * L.lb[2] * INV_2PI_R;
+      G.w = L.w;
+      G.flat = R[2] == 0.0 && R[5] == 0.0 && L.la[2] == 0.0;
+      G.keep = e > (long)ga * a.nscale &&
+               (e % a.nscale != 0 || same_elements<SHAPE>(a, elems, elem_rot + 9 * (long)g * a.nelem));
+    }
+    __syncthreads();
+    for (int j = 0; j < ne; ++j) {
+      const GrainAngles& G = s_g[j];
+      if (!G.keep) {
+        const long g = (e0 + j) / a.nscale;
+        grain_terms<T, SHAPE>(a, shapes, elems, elem_rot + 9 * g * a.nelem, qx, qy, qz, ii, f);
+      }
+      cx<T> sum{0, 0};
+      T ab = 1;
       if (a.sfbuf) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) sum += f[k] * zd(a.sfbuf[k * a.n + i]);
-      } else if (flat && L.la[2] == 0.0) {
-        const Ratio ra = dirichlet_real((p0 * L.la[0] + p1 * L.la[1]) * INV_2PI_R, L.rep[0]);
-        const Ratio rb = dirichlet_real((p0 * L.lb[0] + p1 * L.lb[1] + L.lb[2] * L.lb[2]) * INV_2PI_R, L.rep[1]);
-        ab = (ra.num * rb.num) / (ra.den * rb.den);
-        const double tc = p0 * L.lc[0] + p1 * L.lc[1] + p2 * L.lc[2], zc = gp[8] * L.lc[2];
-#pragma unroll
         for (int k = 0; k < 4; ++k) {
-          zd v = f[k];
-          if (L.rep[2] != 1.0) {
-            const Ratio rc = dirichlet_real((tc + zc * qz[k]) * INV_2PI_R, L.rep[2]);
-            v = v * (rc.num / rc.den);
-          }
-          if (cz != 0.0) v = v * expi_real(gp[8] * qz[k] * cz);  // the rest of the phase is common
-          sum += v;
+          const double2 v = a.sfbuf[k * a.n + ii];
+          sum = sum + f[k] * cx<T>{(T)v.x, (T)v.y};
         }
+      } else if (G.flat) {
+        const Ratio<T> ra = dirichlet_real<T>(fma(qx, G.a[0], qy * G.a[1]), G.rep[0]);
+        const Ratio<T> rb = dirichlet_real<T>(fma(qx, G.b[0], fma(qy, G.b[1], G.b0)), G.rep[1]);
+        ab = quotient(ra.num * rb.num, ra.den * rb.den);
+        cx<T> v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = f[k];
+        if (G.rep[2] != 1.0) {
+          const double tc = fma(qx, G.c[0], qy * G.c[1]);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const Ratio<T> rc = dirichlet_real<T>(fma(qz[k], G.c[2], tc), G.rep[2]);
+            v[k] = quotient(rc.num, rc.den) * v[k];
+          }
+        }
+        if (G.d[2] != 0.0)  // the rest of the centre's phase is common
+#pragma unroll
+          for (int k = 0; k < 4; ++k) v[k] = v[k] * expi_turns_real<T>(qz[k] * G.d[2]);
+        sum = (v[0] + v[1]) + (v[2] + v[3]);
       } else {
 #pragma unroll 1
         for (int k = 0; k < 4; ++k) {
           const double q = k == 0 ? qz[0] : k == 1 ? qz[1] : k == 2 ? qz[2] : qz[3];
-          const zd fk = k == 0 ? f[0] : k == 1 ? f[1] : k == 2 ? f[2] : f[3];
-          const double m0 = p0 + gp[2] * q, m1 = p1 + gp[5] * q, m2 = p2 + gp[8] * q;
-          const double ub = (m0 * L.lb[0] + m1 * L.lb[1] + L.lb[2] * L.lb[2]) * INV_2PI_R;
-          const Ratio ra = dirichlet_real((m0 * L.la[0] + m1 * L.la[1] + m2 * L.la[2]) * INV_2PI_R, L.rep[0]);
-          const Ratio rb = dirichlet_real(ub, L.rep[1]);
-          const Ratio rc = dirichlet_real((m0 * L.lc[0] + m1 * L.lc[1] + m2 * L.lc[2]) * INV_2PI_R, L.rep[2]);
-          zd v = fk * (ra.num * rb.num * rc.num / (ra.den * rb.den * rc.den));
-          if (L.rep[1] != round_fp64(L.rep[1])) v = v * dirichlet_b_phase(ub, L.rep[1]);
-          if (!centred) v = v * expi_real(m0 * cx + m1 * cyy + m2 * cz);
-          sum += v;
+          const cx<T> fk = k == 0 ? f[0] : k == 1 ? f[1] : k == 2 ? f[2] : f[3];
+          const double ub = fma(qx, G.b[0], fma(qy, G.b[1], fma(q, G.b[2], G.b0)));
+          const Ratio<T> ra = dirichlet_real<T>(fma(qx, G.a[0], fma(qy, G.a[1], q * G.a[2])), G.rep[0]);
+          const Ratio<T> rb = dirichlet_real<T>(ub, G.rep[1]);
+          const Ratio<T> rc = dirichlet_real<T>(fma(qx, G.c[0], fma(qy, G.c[1], q * G.c[2])), G.rep[2]);
+          cx<T> v = (quotient(ra.num, ra.den) * quotient(rb.num, rb.den) * quotient(rc.num, rc.den)) * fk;
+          if (G.rep[1] != round_fp64(G.rep[1])) v = v * expi_turns_real<T>(0.5 * round_fp64(ub) * (G.rep[1] - 1.0));
+          if (G.d[0] != 0.0 || G.d[1] != 0.0 || G.d[2] != 0.0)
+            v = v * expi_turns_real<T>(fma(qx, G.d[0], fma(qy, G.d[1], q * G.d[2])));
+          sum = sum + v;
         }
       }
-      const double w = L.w * ab;
-      acc += w * w * (sum.x * sum.x + sum.y * sum.y);
+      const T w = (T)G.w * ab;
+      acc += (double)(w * w * (sum.x * sum.x + sum.y * sum.y));
     }
   }
-  out[i] = acc;
+  if (live) out[i] = acc;
 }
 
 // out += the splits' sums, in order.
@@ -480,24 +446,17 @@ __global__ void grain_sum_kernel(const double* __restrict__ part, int splits, lo
   out[i] = v;
 }
 
-// true when the real-qz grain kernels (FP32C and FP64) have a body for this shape
-static bool grain_f32c_shape(int shape) {
+// true when the real-qz grain kernel has a body for this shape
+static bool grain_real_shape(int shape) {
   return shape == SH_CYLINDER || shape == SH_SPHERE || shape == SH_BOX;
 }
 
+template <typename T>
 static void launch_grain_real(int shape, dim3 grid, cudaStream_t st, const FusedArgs& a) {
   switch (shape) {
-    case SH_CYLINDER: grain_dwba_real_kernel<SH_CYLINDER><<<grid, 128, 0, st>>>(a); break;
-    case SH_SPHERE: grain_dwba_real_kernel<SH_SPHERE><<<grid, 128, 0, st>>>(a); break;
-    default: grain_dwba_real_kernel<SH_BOX><<<grid, 128, 0, st>>>(a); break;
-  }
-}
-
-static void launch_grain_f32c(int shape, unsigned blocks, cudaStream_t st, const FusedArgs& a) {
-  switch (shape) {
-    case SH_CYLINDER: grain_dwba_f32c_kernel<SH_CYLINDER><<<blocks, 128, 0, st>>>(a); break;
-    case SH_SPHERE: grain_dwba_f32c_kernel<SH_SPHERE><<<blocks, 128, 0, st>>>(a); break;
-    default: grain_dwba_f32c_kernel<SH_BOX><<<blocks, 128, 0, st>>>(a); break;
+    case SH_CYLINDER: grain_dwba_real_kernel<T, SH_CYLINDER><<<grid, 128, 0, st>>>(a); break;
+    case SH_SPHERE: grain_dwba_real_kernel<T, SH_SPHERE><<<grid, 128, 0, st>>>(a); break;
+    default: grain_dwba_real_kernel<T, SH_BOX><<<grid, 128, 0, st>>>(a); break;
   }
 }
 
@@ -1075,9 +1034,8 @@ static int fused_structure(hgx_ctx c, hgx_qgrid g, HigWork& w, const hig::Struct
   int one = nelem > 0 ? shapes[0].shape : 0;  // the shape every element shares, if any
   for (int e = 1; e < nelem; ++e)
     if (shapes[e].shape != one) one = 0;
-  // FP32C: grids with real qz blocks (paired rows) and one shape with an FP32C body
-  const bool f32c = precision == HGX_F32C && g->mode == 1 && grain_f32c_shape(one);
-  if (!f32c && g->mode == 1 && grain_f32c_shape(one)) {
+  // grids with real qz blocks (paired rows) and one shape with a real-qz body
+  if (g->mode == 1 && grain_real_shape(one)) {
     const unsigned blocks1 = (unsigned)((a.n + 127) / 128);
     // four CTAs of 128 threads run per SM; grains are split where the pixels do not fill them
     const int splits = (int)std::max<long>(1, std::min<long>({4L * c->sm_count / blocks1, (long)ngr / 4, 32}));
@@ -1088,7 +1046,8 @@ static int fused_structure(hgx_ctx c, hgx_qgrid g, HigWork& w, const hig::Struct
     for (int g0 = 0; g0 < ngr; g0 += REAL_GRAINS_PER_LAUNCH) {
       a.g0 = g0;
       a.g1 = std::min(ngr, g0 + REAL_GRAINS_PER_LAUNCH);
-      launch_grain_real(one, dim3(blocks1, 1, splits), st, a);
+      if (precision == HGX_F32C) launch_grain_real<float>(one, dim3(blocks1, 1, splits), st, a);
+      else launch_grain_real<double>(one, dim3(blocks1, 1, splits), st, a);
       if (splits > 1) grain_sum_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a.part, splits, a.n, a.out);
       HGX_CUDA(cudaGetLastError());
     }
@@ -1097,11 +1056,6 @@ static int fused_structure(hgx_ctx c, hgx_qgrid g, HigWork& w, const hig::Struct
   for (int g0 = 0; g0 < ngr; g0 += FUSED_GRAINS_PER_LAUNCH) {
     a.g0 = g0;
     a.g1 = g0 + FUSED_GRAINS_PER_LAUNCH < ngr ? g0 + FUSED_GRAINS_PER_LAUNCH : ngr;
-    if (f32c) {
-      launch_grain_f32c(one, blocks, st, a);
-      HGX_CUDA(cudaGetLastError());
-      continue;
-    }
     // the paired lattice factor when it holds for every grain and sample of the launch
     bool paired = a.sfbuf == nullptr;
     for (int gi = a.g0; gi < a.g1 && paired; ++gi) {
@@ -1700,8 +1654,8 @@ namespace {
 // one structure's per-candidate table sizes and its launch choices
 struct PopStruct {
   int ngr = 0, nscale = 0, nelem = 0, shape = 0;
-  bool liquid = false, f32c = false;
-  bool real = false;  // FP64 on real qz: grain_dwba_real_kernel
+  bool liquid = false;
+  bool real = false, f32c = false;  // grain_dwba_real_kernel, its precision
   // byte offsets in the staging block of each table's region; a region holds the table of every
   // candidate in turn (candidate i at i x the table's size)
   size_t o_shapes = 0, o_elems = 0, o_gt = 0, o_er = 0, o_sc = 0;
@@ -1818,13 +1772,9 @@ int pop_enqueue(hgx_hig_pop_s& P, cudaStream_t st) {
       a.g0 = g0;
       a.g1 = std::min(ps.ngr, g0 + chunk);
       if (ps.real) {
-        launch_grain_real(ps.shape, dim3((unsigned)((n + 127) / 128), (unsigned)P.npop), st, a);
-      } else if (ps.f32c) {
-        switch (ps.shape) {
-          case SH_CYLINDER: grain_dwba_f32c_kernel<SH_CYLINDER><<<grid, 128, 0, st>>>(a); break;
-          case SH_SPHERE: grain_dwba_f32c_kernel<SH_SPHERE><<<grid, 128, 0, st>>>(a); break;
-          default: grain_dwba_f32c_kernel<SH_BOX><<<grid, 128, 0, st>>>(a); break;
-        }
+        const dim3 g1((unsigned)((n + 127) / 128), (unsigned)P.npop);
+        if (ps.f32c) launch_grain_real<float>(ps.shape, g1, st, a);
+        else launch_grain_real<double>(ps.shape, g1, st, a);
       } else {
         const int paired = P.variants[vi++];
 #define HGX_POP_LAUNCH(S)                                                   \
@@ -1960,8 +1910,8 @@ int hgx_hig_population_create(hgx_ctx c, hgx_hig h, int npop, const double* ref,
     ps.nelem = (int)t.f.elems.size();
     ps.shape = t.shape;
     ps.liquid = t.liquid;
-    ps.f32c = precision == HGX_F32C && g->mode == 1 && grain_f32c_shape(t.shape);
-    ps.real = !ps.f32c && g->mode == 1 && grain_f32c_shape(t.shape);
+    ps.f32c = precision == HGX_F32C;
+    ps.real = g->mode == 1 && grain_real_shape(t.shape);
     ps.n_gt = t.f.gt.size();
     ps.n_er = t.f.er.size();
     ps.n_sc = t.plan.size();
@@ -2047,7 +1997,7 @@ int hgx_hig_population_eval(hgx_hig_pop p, const double* X, int nx, double* dist
   const int chunk = pop_chunk(p->npop);
   for (int k = 0; k < p->nstruct; ++k) {
     const PopStruct& ps = p->st[k];
-    if (ps.f32c || ps.real) continue;
+    if (ps.real) continue;
     for (int g0 = 0; g0 < ps.ngr; g0 += chunk) v.push_back(pop_paired(all, k, g0, std::min(ps.ngr, g0 + chunk)));
   }
   if (p->exec && v != p->variants) {  // another kernel variant: record the graph again

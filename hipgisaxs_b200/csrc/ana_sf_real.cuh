@@ -54,14 +54,9 @@ __device__ __forceinline__ cx<float> expi_turns_real<float>(double u) {
 template <typename T>
 __device__ __forceinline__ cx<T> expi_real(double ph) { return expi_turns_real<T>(ph * INV_2PI_R); }
 
-// sin(x) / x (hig::sinc for a real x) given sin x
-__device__ __forceinline__ double sinc_real(double x, double sinx) {
-  return fabs(x) > 1.0e-14 ? sinx / x : 1.0;
-}
-__device__ __forceinline__ float sinc_real(double x, float sinx) { return sinc_from(x, sinx); }
-
 // a / b.  FP64: b's reciprocal by two Newton steps from the FP32 approximation (23 bits), without
-// the branches of the IEEE division; within two ulp for 1e-37 < |b| < 1e37 (sines here).
+// the branches of the IEEE division; within two ulp for 1e-37 < |b| < 1e37
+// (sines and phases here).
 __device__ __forceinline__ double quotient(double a, double b) {
   float y0;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"((float)b));
@@ -71,6 +66,12 @@ __device__ __forceinline__ double quotient(double a, double b) {
   return a * y;
 }
 __device__ __forceinline__ float quotient(float a, float b) { return __fdividef(a, b); }
+
+// sin(x) / x (hig::sinc for a real x) given sin x
+__device__ __forceinline__ double sinc_real(double x, double sinx) {
+  return fabs(x) > 1.0e-14 ? quotient(sinx, x) : 1.0;
+}
+__device__ __forceinline__ float sinc_real(double x, float sinx) { return sinc_from(x, sinx); }
 
 // A lattice factor as num / den at the angle of `u` turns; N itself within 1e-13 turn of a whole
 // one, where the ratio is N to rounding (the products of two denominators then stay in range).
@@ -105,7 +106,7 @@ static __device__ __noinline__ T cyl_radial_real(const Dist& X, double qpar) {
   for (int i = 0; i < X.n; ++i) {
     const double r = X.v[i], x = qpar * r;
     if (x * x > CUTINY_REF) {
-      if (sizeof(T) == 8) fr += (T)(j1(x) / x * (2. * PI_REF * r * r));
+      if (sizeof(T) == 8) fr += (T)(quotient(j1(x), x) * (2. * PI_REF * r * r));
       else fr += (T)((float)(2. * PI_REF * r * r) * (j1f((float)x) / (float)x));
     }
   }

@@ -48,35 +48,28 @@ __device__ void parratt(const Stack& S, double alpha, double k0, zd* T_out, zd* 
   *R_out = R[S.order] / t0;
 }
 
-// One thread per detector row: Tf, Rf (zero when alpha_f <= 0); thread 0 of block 0 also
-// writes the incident coefficients into slot nrow.
-__global__ void parratt_rows_kernel(Stack S, const double* __restrict__ alpha, int nrow,
-                                    double alpha_i, double k0, double2* __restrict__ tr) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < nrow) {
-    zd T(0, 0), R(0, 0);
-    if (alpha[r] > 0) parratt(S, alpha[r], k0, &T, &R);
-    tr[2 * r] = T.d2();
-    tr[2 * r + 1] = R.d2();
+// Per-row DWBA coefficients rowfc[r*4 + k]: one thread per detector row (Tf = Rf = 0 when alpha_f
+// <= 0); the last thread of each block makes the incident amplitudes for the block's rows.
+constexpr int FC_ROWS = 63;
+__global__ void __launch_bounds__(FC_ROWS + 1) parratt_rows_kernel(Stack S, const double* __restrict__ alpha, int nrow,
+                                                                  double alpha_i, double k0, double2* __restrict__ rowfc) {
+  __shared__ zd s_i[2];
+  const int r = blockIdx.x * FC_ROWS + threadIdx.x;
+  const bool incident = threadIdx.x == FC_ROWS, mine = !incident && r < nrow;
+  zd T(0, 0), R(0, 0);
+  const double al = incident ? alpha_i : mine ? alpha[r] : 0.0;
+  if (incident || al > 0) parratt(S, al, k0, &T, &R);
+  if (incident) {
+    s_i[0] = T;
+    s_i[1] = R;
   }
-  if (r == 0) {
-    zd T, R;
-    parratt(S, alpha_i, k0, &T, &R);
-    tr[2 * nrow] = T.d2();
-    tr[2 * nrow + 1] = R.d2();
-  }
-}
-
-// Per-row DWBA coefficients: rowfc[r*4 + k].
-__global__ void row_fc_kernel(const double2* __restrict__ tr, int nrow, double2* __restrict__ rowfc) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nrow) return;
-  zd Ti(tr[2 * nrow]), Ri(tr[2 * nrow + 1]);
-  zd Tf(tr[2 * r]), Rf(tr[2 * r + 1]);
-  rowfc[4 * r + 0] = (Ti * conj(Tf)).d2();
-  rowfc[4 * r + 1] = (Ti * conj(Rf)).d2();
-  rowfc[4 * r + 2] = (Ri * conj(Tf)).d2();
-  rowfc[4 * r + 3] = (Ri * conj(Rf)).d2();
+  __syncthreads();
+  if (!mine) return;
+  const zd Ti = s_i[0], Ri = s_i[1];
+  rowfc[4 * r + 0] = (Ti * conj(T)).d2();
+  rowfc[4 * r + 1] = (Ti * conj(R)).d2();
+  rowfc[4 * r + 2] = (Ri * conj(T)).d2();
+  rowfc[4 * r + 3] = (Ri * conj(R)).d2();
 }
 
 // Expands per-row coefficients to the reference's per-pixel 4N layout.
@@ -136,14 +129,9 @@ int build_stack(int nlayers, const double* delta, const double* beta, const doub
 // Per-row coefficients (nrow x 4 complex128) into `rowfc` (device).
 int row_fc_device(hgx_ctx c, const Stack& S, const double* alpha_dev, int nrow, double k0,
                   double alpha_i, double2* rowfc) {
-  DevBuf tr;
-  HGX_TRY(tr.reserve(sizeof(double2) * 2 * (size_t)(nrow + 1)));
-  parratt_rows_kernel<<<(nrow + 63) / 64, 64, 0, c->stream>>>(S, alpha_dev, nrow, alpha_i, k0,
-                                                              reinterpret_cast<double2*>(tr.p));
-  row_fc_kernel<<<(nrow + 127) / 128, 128, 0, c->stream>>>(reinterpret_cast<double2*>(tr.p), nrow,
-                                                           rowfc);
+  parratt_rows_kernel<<<(nrow + FC_ROWS - 1) / FC_ROWS, FC_ROWS + 1, 0, c->stream>>>(S, alpha_dev, nrow, alpha_i, k0,
+                                                                                    rowfc);
   HGX_CUDA(cudaGetLastError());
-  HGX_CUDA(cudaStreamSynchronize(c->stream));  // `tr` is released on return
   return HGX_OK;
 }
 
@@ -167,7 +155,7 @@ int hgx_propagation_coeffs(hgx_ctx c, hgx_qgrid g, int nlayers, const double* de
   const double* al = alpha ? alpha : g->alpha;
   if (!al)
     return fail(HGX_ERR_INVALID_ARG, "hgx_propagation_coeffs: exit angles needed (grid from arrays)");
-  DevBuf abuf, rowbuf, outbuf;
+  DevBuf abuf, outbuf;
   const void* al_dev = nullptr;
   HGX_TRY(stage_in(c, al, sizeof(double) * g->nrow, abuf, &al_dev));
   const long n = (long)g->nrow * g->ncol;
@@ -176,8 +164,8 @@ int hgx_propagation_coeffs(hgx_ctx c, hgx_qgrid g, int nlayers, const double* de
   HGX_TRY(stage_out(c, fc, out_bytes, outbuf, &dout));
   double2* rowfc = reinterpret_cast<double2*>(dout);
   if (!per_row) {
-    HGX_TRY(rowbuf.reserve(sizeof(double2) * 4 * (size_t)g->nrow));
-    rowfc = reinterpret_cast<double2*>(rowbuf.p);
+    HGX_TRY(c->rowfc.reserve(sizeof(double2) * 4 * (size_t)g->nrow));
+    rowfc = reinterpret_cast<double2*>(c->rowfc.p);
   }
   HGX_TRY(row_fc_device(c, S, reinterpret_cast<const double*>(al_dev), g->nrow, k0, alpha_i, rowfc));
   if (!per_row) {

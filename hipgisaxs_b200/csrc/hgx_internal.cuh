@@ -134,6 +134,7 @@ struct hgx_ctx_s {
   unsigned* d_err = nullptr;  // device error word (DeviceError bits)
   hgx::DevBuf scratch;        // per-call scratch, grown on demand
   hgx::DevBuf factors;        // row factors and partial sums of the tensor-core row kernel
+  hgx::DevBuf rowfc;          // per-row Fresnel coefficients on their way to the per-pixel layout
   hgx::TileView tiles;        // triangle tiles of the last FP32C form factor (in scratch)
   hgx::DevBuf staging;        // device copies of host inputs
   int sm_count = 148;

@@ -700,13 +700,13 @@ static int run(hgx_ctx c, hgx_qgrid g, const MmaTiles& t, const Rot9& R, void* o
     const long full = rows * ncoltiles / wave * wave / ncoltiles;
     if (full > 0) rows = full;
   } else {
-    // few items: the tiles are split over CTAs where that fills the last wave better; an
-    // item's own cost (its first fetch, the partial sums) is taken as 0.3 of a tile
+    // few items: the tiles are split over CTAs where that fills the last wave better; an item's own
+    // cost (its start, first fetch and end) is about a tile's, and so is adding the splits' sums
     const long items = rows * ncoltiles;
     const size_t part = (size_t)rows * g->ncol * S::NACC * sizeof(double);
     double best = 0.0;
     for (int k = 1; k <= t.ntiles && k <= 32 && (k == 1 || k * part <= PART_BYTES); ++k) {
-      const double cost = (double)((items * k + wave - 1) / wave) * ((t.ntiles + k - 1) / k + 0.3);
+      const double cost = (double)((items * k + wave - 1) / wave) * ((t.ntiles + k - 1) / k + 1.0) + (k > 1);
       if (k == 1 || cost < best) {
         best = cost;
         nsplit = k;

@@ -66,6 +66,15 @@ def test_slabs_of_row_factors(ctx, po):
     assert po.rel_err(hg.ff_triangles(ctx, g, sd, None, "f32c"), f64) < TOL32
 
 
+@pytest.mark.parametrize("ntri", [514, 1024, 1025, 2048, 2049])
+def test_order_of_small_and_large_meshes(ctx, po, ntri):
+    """Both ways of ordering the triangles, at the line between them."""
+    sd = cloud(np.random.default_rng(ntri), ntri)
+    qx, qy, qz = detector(po, 20, 2, "real")
+    g = hg.QGrid.from_arrays(ctx, qx, qy, qz, 20)
+    assert po.rel_err(hg.ff_triangles(ctx, g, sd, None, "f32c"), po.ff_approx_triangle(sd, qx, qy, qz)) < TOL32
+
+
 @pytest.mark.parametrize("col,value", [(0, np.nan), (0, np.inf), (2, np.nan), (5, np.nan), (6, np.inf)])
 def test_a_triangle_that_is_not_finite_is_not_hidden(ctx, po, col, value):
     sd = cloud(np.random.default_rng(6), 600)

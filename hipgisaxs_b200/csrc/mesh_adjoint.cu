@@ -22,6 +22,8 @@
 // with E = e^{i(qx c'x + qy c'y)} and A = qx n~'x + qy n~'y in the rotated frame.  Per-chunk
 // partial gradients are summed in a fixed order (deterministic), rotated back, and chained
 // to the vertices: n~ = (v2 - v1) x (v3 - v1) / 2, c = (v1 + v2 + v3)/3.
+// FP32C on grids wider than 128 columns takes the sums over pixels to the tensor cores
+// (mesh_adjoint_mma.cu); the FP32 kernel here serves narrower ones.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -30,6 +32,7 @@
 
 #include "cplx.cuh"
 #include "hgx_internal.cuh"
+#include "mesh_adjoint.cuh"
 
 namespace hgx {
 
@@ -570,11 +573,24 @@ int hgx_mesh_chi2_grad_ex(hgx_ctx c, hgx_qgrid g, int nv, const double* verts, i
     const TileView tv = c->tiles;
     if (!f64 && (tv.ntri != nf || !tv.perm))
       return fail(HGX_ERR_INVALID_ARG, "hgx_mesh_chi2_grad: the forward left no triangle tiles");
+    const BwmPlan plan = f64 ? BwmPlan{} : bwm_plan(c, g, tv.ntiles, nf);
     const int ntile = f64 ? (nf + BW_TRI - 1) / BW_TRI : tv.ntiles;
     int chunks = std::max(1, (c->sm_count * 16) / std::max(1, ntile));
     chunks = std::min(chunks, g->nrow);
     const int rpc = (g->nrow + chunks - 1) / chunks;
     chunks = (g->nrow + rpc - 1) / rpc;
+    int done = HGX_ERR_NO_MEMORY;
+    if (plan.slabs) {
+      // every slab has the same number of row ranges; the last one may have fewer rows than ranges
+      const int parts = plan.slabs * plan.splits;
+      HGX_TRY(w.bwpart.reserve(sizeof(double) * 6 * (size_t)nf * std::max(parts, chunks)));
+      HGX_CUDA(cudaMemsetAsync(w.bwpart.p, 0, sizeof(double) * 6 * (size_t)nf * parts, st));
+      BwmArgs ba{tv.tiles, tv.anchors, tv.perm, nf, tv.ntiles, (const float4*)seeds.p, g->qx, g->qy, g->rowqz,
+                 g->nrow, g->ncol, (double*)w.bwpart.p};
+      done = bwm_run(c, plan, ba);
+      if (done == HGX_OK) chunks = parts;
+      else if (done != HGX_ERR_NO_MEMORY) return done;  // without room for the seed digits: the FP32 kernel
+    }
     HGX_TRY(gtri.reserve(sizeof(double) * 6 * nf));
     DevBuf& bwpart = w.bwpart;
     HGX_TRY(bwpart.reserve(sizeof(double) * 6 * (size_t)nf * chunks));
@@ -593,7 +609,7 @@ int hgx_mesh_chi2_grad_ex(hgx_ctx c, hgx_qgrid g, int nv, const double* verts, i
       ba.rows_per_chunk = rpc;
       ba.partial = (double*)bwpart.p;
       mesh_backward_f64_kernel<<<grid, BW_THREADS, 0, st>>>(ba);
-    } else {
+    } else if (done != HGX_OK) {
       BwArgs ba;
       ba.tiles = tv.tiles;  // tiles left by the forward
       ba.anchors = tv.anchors;

@@ -43,9 +43,10 @@ int param_distribution_host(int stat, double pmin, double pmax, double mean, dou
                             int nvalues, std::vector<double>& dim, std::vector<double>& w);
 
 constexpr int CYL_MAXS = 64;
-constexpr int CYL_THREADS = 256;                   // block of the row-table and final kernels
+constexpr int CYL_THREADS = 1024;                  // block of the final kernel
 // Tile shapes of the persistent pixel pass: threads per block x pixels per thread; one work
-// item is one tile of threads*ppt consecutive ROI pixels.  Shape 0 is the default; the
+// item is one tile of threads*ppt consecutive ROI pixels (FP64; FP32C cuts its tiles into
+// warps' items of at most ppt pixels per lane).  Shape 0 is the default; the
 // autotuner (hgx_cyl_batch_tune) times all of them on the batch's own ROIs.
 struct CylShape {
   int threads, ppt;
@@ -69,29 +70,52 @@ constexpr double PI_D = 3.141592653589793;
 enum { M_R = 0, M_H = 1, M_A = 2, M_PHI = 3, M_SPREAD = 4, M_NSAMP = 5, M_REP = 6, M_DN2 = 9,
        M_CENTER = 11, M_WEIGHT = 14, M_SAMPLING = 15 };
 
+// What the FP32C pixel pass reads of a candidate per pixel; a block copies it to shared memory in
+// 16-byte words (from global memory its 20 fields were 20 loads per pixel, as the stores could alias them).
+struct alignas(16) CylPix {
+  double cphi, sphi;
+  double ka[2], kb[2];      // a ua / 2pi, a ub / 2pi: lattice phases in turns
+  double rep[2];
+  double scale, qmin2;      // below |q_par|^2 = qmin2 some radius meets the q_par -> 0 guard
+  float fu0[2], fu1[2];     // x and y of ua, ub
+  float fa, fscale, frep[2];
+  float ser[2][8];          // Dirichlet series of the a- and b-directions (cyl_dirichlet_series)
+  float lim[2], pad[2];     // and where they are used (dirichlet_pair)
+  long px_off, rowtab0;     // the layout fields of CylCand
+  int row0, col0, nrows, ncols;
+  int per_lane;             // pixels per lane and item
+  int dq, dr, pad2;         // 32 pixels on in the region: dq rows and dr columns
+};
+static_assert(sizeof(CylPix) == 240, "copied in 16-byte words");
+
 struct CylCand {
+  CylPix pix;
   double R, H, a, cphi, sphi;
   double rep[3];
   double K[2];       // weight * dn2
   double center[3];
   double ua[2], ub[2], uc;  // unscaled lattice vectors (in-plane a, b; c along z)
-  double ka[2], kb[2];      // a ua / 2pi, a ub / 2pi: lattice phases in turns
-  float ser[2][8];          // FP32C Dirichlet series of the a- and b-directions (cyl_dirichlet_series)
-  float fa, fua[2], fub[2], frep[2], fscale;  // FP32 copies for the FP32C pixel pass
   int nr, nh;
   int row0, col0, nrows, ncols;
   long px_off;       // offset of this candidate's pixels in counts / intensity
   long item0, nitems;
   long rowtab0;      // offset of this candidate's rows in the row table
   double scale;
-  double rmin;       // smallest radius sample (the q_par -> 0 guard of the radial sums)
   double r[CYL_MAXS];
   double h[CYL_MAXS];
 };
 
-struct RowTab {
-  double q2, qh, qa;     // |K Q|^2, |K|^2 Re(conj(Q) dQ/dH), |K|^2 Re(conj(Q) dQ/da)
-  float q2f, qhf, qaf;   // the same rounded to FP32 (the FP32C derivative products)
+struct alignas(16) RowTab {
+  double q2;             // |K Q|^2
+  float q2f, qhf;        // q2 and qh rounded to FP32 (the FP32C derivative products)
+  float qaf;
+  double qh, qa;         // |K|^2 Re(conj(Q) dQ/dH), |K|^2 Re(conj(Q) dQ/da)
+};
+
+// One interval of the radial-sum tables: the cubics of fr and frR / R and their constant terms' rests.
+struct CylCell {
+  float4 fr, frR;
+  float2 lo, pad;
 };
 
 // S_N(theta) = sin(N pi t)/sin(pi t), t = theta/2pi reduced, and dS/dtheta (FP64).
@@ -122,33 +146,34 @@ __device__ __forceinline__ void dirichlet(double theta, double N, double* S, dou
   *dS = (N * cn * s1 - sn * c1) / (2.0 * s1 * s1);
 }
 
-// The Dirichlet kernel in FP32 arithmetic at a turn t already reduced to [-1/2, 1/2] in FP64.
-// N t is reduced modulo 2 in FP64 too (sin and cos of pi N t keep their values), so both sines
-// keep FP32 accuracy for any N.  For |theta| N < 1 the closed form's derivative cancels; there
-// the series in y = (theta N)^2 with the candidate's scaled power sums: e[0..3] for S, e[4..7]
-// for dS.
-__device__ __forceinline__ void dirichlet_f32(double t, double N, float Nf, const float* e,
-                                              float* S, float* dS) {
-  if (N == 1.0) {
-    *S = 1.0f;
-    *dS = 0.0f;
-    return;
+// The Dirichlet kernels of the a- and b-directions in FP32 arithmetic, two to an FP32x2 operation, at
+// turns t already reduced to [-1/2, 1/2] in FP64.  N t is reduced modulo 2 in FP64 too (sin and
+// cos of pi N t keep their values), so both sines keep FP32 accuracy for any N.  For |theta| N <
+// lim = 1 the closed form's derivative cancels; there the series in y = (theta N)^2 with the
+// candidate's scaled power sums: e[0..3] for S, e[4..7] for dS.  N = 1: lim is infinite and the
+// sums are 0, so S = 1 and dS = 0 everywhere.
+__device__ __forceinline__ void dirichlet_pair(double ta, double tb, const CylPix& k, float2* S, float2* dS) {
+  const double ua = k.rep[0] * ta, ub = k.rep[1] * tb;
+  const float2 tf = make_float2((float)ta, (float)tb), N = make_float2(k.frep[0], k.frep[1]);
+  const float2 thN = __fmul2_rn(__fmul2_rn(make_float2(6.28318530718f, 6.28318530718f), tf), N);
+  float2 sn, cn, s1, c1;
+  sincospi_f32x2(make_float2((float)(ua - 2.0 * round_fp64(0.5 * ua)), (float)(ub - 2.0 * round_fp64(0.5 * ub))), &sn,
+                 &cn);
+  sincospi_f32x2(tf, &s1, &c1);
+  const float2 inv = make_float2(__frcp_rn(s1.x), __frcp_rn(s1.y));
+  *S = __fmul2_rn(sn, inv);
+  const float2 d = __ffma2_rn(make_float2(-S->x, -S->y), c1, __fmul2_rn(N, cn));
+  *dS = __fmul2_rn(__fmul2_rn(make_float2(0.5f, 0.5f), d), inv);
+  if (fabsf(thN.x) < k.lim[0] || fabsf(thN.y) < k.lim[1]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float th = i ? thN.y : thN.x, n = i ? N.y : N.x, y = th * th, *e = k.ser[i];
+      if (fabsf(th) < k.lim[i]) {
+        (i ? S->y : S->x) = n * (1.0f - y * (e[0] - y * (e[1] - y * (e[2] - y * e[3]))));
+        (i ? dS->y : dS->x) = -th * n * n * (e[4] - y * (e[5] - y * (e[6] - y * e[7])));
+      }
+    }
   }
-  const float tf = (float)t;
-  const float thN = 6.28318530718f * tf * Nf;
-  if (fabsf(thN) < 1.0f) {
-    const float y = thN * thN;
-    *S = Nf * (1.0f - y * (e[0] - y * (e[1] - y * (e[2] - y * e[3]))));
-    *dS = -thN * Nf * Nf * (e[4] - y * (e[5] - y * (e[6] - y * e[7])));
-    return;
-  }
-  const double u = N * t;
-  float sn, cn, s1, c1;
-  sincospi_f32((float)(u - 2.0 * round_fp64(0.5 * u)), &sn, &cn);
-  sincospi_f32(tf, &s1, &c1);
-  const float inv = __frcp_rn(s1), Sv = sn * inv;
-  *S = Sv;
-  *dS = 0.5f * (Nf * cn - Sv * c1) * inv;
 }
 
 // ---------------------------------------------------------------- row table ----
@@ -211,38 +236,58 @@ __device__ __forceinline__ void cyl_rows_body(const CylCand& c, int bx, const do
 }
 
 // --------------------------------------------------------- radial-sum tables ----
-// 8 lanes per node: lane l sums the radius samples l, l + 8, ..., xor shuffles close the sum
-// ((fr, frR) at q = |j - 1| h, as the pixel pass would sum them), except that the q_par -> 0
-// guard takes the smooth limit (J1(x)/x -> 1/2, J0 -> 1) so that the interpolation near q = 0
-// is right; pixels that meet the guard sum directly.  Each FP64 sum is stored as an FP32 pair
-// (hi, lo = sum - hi): the pixel pass interpolates both in FP32, so no rounding of a node,
-// common to every pixel near that q_par, reaches the intensity.
-__device__ __forceinline__ void cyl_table_body(const CylCand& c, int bx, double h, float4* __restrict__ table) {
-  const int j = (int)((bx * blockDim.x + threadIdx.x) >> 3), l = threadIdx.x & 7;
+// A block sums 32 nodes, 8 lanes per node: lane l takes the radius samples l, l + 8, ..., xor
+// shuffles close the sum ((fr, frR) at q = |j - 1| h, as the pixel pass would sum them), except
+// that the q_par -> 0 guard takes the smooth limit (J1(x)/x -> 1/2, J0 -> 1) so that the
+// interpolation near q = 0 is right; pixels that meet the guard sum directly.  Then 29 threads
+// make the cubics of the intervals from node j0 + 1 on: the polynomial in t of the 4-point
+// Lagrange interpolation (nodes at t = -1, 0, 1, 2), in FP64 and rounded to FP32, with the constant term as
+// a pair (hi, lo), so that no rounding of a node, common to every pixel near that q_par, reaches
+// the intensity (the other terms vanish at the nodes and are a few per cent of it between them).
+constexpr int CYL_PREP_THREADS = 256;
+constexpr int CYL_CELLS = CYL_PREP_THREADS / 8 - 3;
+
+__device__ __forceinline__ void cyl_table_body(const CylCand& c, int bx, double h, CylCell* __restrict__ table) {
+  __shared__ double s_node[CYL_PREP_THREADS / 8][2];
+  const int n = threadIdx.x >> 3, l = threadIdx.x & 7, j = bx * CYL_CELLS + n;
   const double qp = fabs((double)(j - 1) * h);
   double fr = 0.0, frR = 0.0;
-  if (j < CYL_NTAB)  // lanes past the last node still join the shuffles
-    for (int i = l; i < c.nr; i += 8) {
-      const double r = c.r[i];
-      const double x = qp * r;
-      const double two_pi_r = 2.0 * PI_D * r;
-      if (x * x > 1.0e-13) {
-        fr += two_pi_r * r * j1(x) / x;
-        frR += two_pi_r * r * j0(x);
-      } else {
-        fr += two_pi_r * r * 0.5;
-        frR += two_pi_r * r;
-      }
+  for (int i = l; i < c.nr; i += 8) {
+    const double r = c.r[i];
+    const double x = qp * r;
+    const double two_pi_r = 2.0 * PI_D * r;
+    if (x * x > 1.0e-13) {
+      fr += two_pi_r * r * j1(x) / x;
+      frR += two_pi_r * r * j0(x);
+    } else {
+      fr += two_pi_r * r * 0.5;
+      frR += two_pi_r * r;
     }
+  }
 #pragma unroll
   for (int o = 1; o < 8; o <<= 1) {
     fr += __shfl_xor_sync(0xffffffffu, fr, o);
     frR += __shfl_xor_sync(0xffffffffu, frR, o);
   }
-  if (j < CYL_NTAB && l == 0) {
-    const double v = frR / c.R;
-    const float fh = (float)fr, vh = (float)v;
-    table[(long)blockIdx.y * CYL_NTAB + j] = make_float4(fh, (float)(fr - fh), vh, (float)(v - vh));
+  if (l == 0) {
+    s_node[n][0] = fr;
+    s_node[n][1] = frR / c.R;
+  }
+  __syncthreads();
+  const int cell = bx * CYL_CELLS + 1 + (int)threadIdx.x;
+  if (threadIdx.x < CYL_CELLS && cell < CYL_NTAB) {
+    float4 f[2];
+    float lo[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const double a = s_node[threadIdx.x][k], b = s_node[threadIdx.x + 1][k], d = s_node[threadIdx.x + 2][k],
+                   e = s_node[threadIdx.x + 3][k];
+      const float hi = (float)b;
+      lo[k] = (float)(b - (double)hi);
+      f[k] = make_float4(hi, (float)(d - 0.5 * b - (2.0 * a + e) / 6.0), (float)(0.5 * (a + d) - b),
+                         (float)(0.5 * (b - d) + (e - a) / 6.0));
+    }
+    table[(long)blockIdx.y * CYL_NTAB + cell] = CylCell{f[0], f[1], make_float2(lo[0], lo[1]), make_float2(0.f, 0.f)};
   }
 }
 
@@ -250,7 +295,7 @@ __device__ __forceinline__ void cyl_table_body(const CylCand& c, int bx, double 
 // per ROI row), the rest (FP32C only) the radial-sum tables; grid y = candidate.
 __global__ void cyl_prep_kernel(const CylCand* __restrict__ cands, int row_blocks,
                                 const double2* __restrict__ rowqz, const double2* __restrict__ rowfc,
-                                RowTab* __restrict__ tab, double h, float4* __restrict__ table) {
+                                RowTab* __restrict__ tab, double h, CylCell* __restrict__ table) {
   const CylCand& c = cands[blockIdx.y];
   if ((int)blockIdx.x < row_blocks)
     cyl_rows_body(c, blockIdx.x, rowqz, rowfc, tab);
@@ -261,7 +306,7 @@ __global__ void cyl_prep_kernel(const CylCand* __restrict__ cands, int row_block
 // --------------------------------------------------------------- pixel pass ----
 struct CylArgs {
   const CylCand* cands;
-  const int2* items;     // (candidate, first pixel of the tile)
+  const int2* items;     // (candidate, first pixel)
   long nitems;
   const RowTab* tab;
   const double* qx;
@@ -271,35 +316,44 @@ struct CylArgs {
   const unsigned* mask;  // may be NULL
   double* intensity;     // may be NULL
   double* partial;       // 5 doubles per item (chi2, dR, dH, da, dphi)
-  const float4* table;   // FP32C: CYL_NTAB (fr hi, lo, frR/R hi, lo) per candidate
+  const CylCell* table;  // FP32C: CYL_NTAB intervals per candidate
   double inv_h;          // 1 / node spacing of the table
   const float* wf;       // FP32C: mask / max(counts, 1) per pixel (may be NULL: forward only)
 };
 
+// v[5] per lane -> the warp's sums, v[warp_slot()] in a lane where that is not negative; fixed order.
+// The shuffles halve the values a lane carries as they halve the lanes (8 exchanges instead of 25).
+__device__ __forceinline__ double warp_sum5(const double* v) {
+  const int lane = threadIdx.x & 31;
+  const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
+  const double a0 = (u16 ? v[3] : v[0]) + __shfl_xor_sync(0xffffffffu, u16 ? v[0] : v[3], 16);
+  const double a1 = (u16 ? v[4] : v[1]) + __shfl_xor_sync(0xffffffffu, u16 ? v[1] : v[4], 16);
+  const double a2 = v[2] + __shfl_xor_sync(0xffffffffu, v[2], 16);
+  const double b0 = (u8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, u8 ? a0 : a1, 8);
+  const double b1 = a2 + __shfl_xor_sync(0xffffffffu, a2, 8);
+  double c = (u4 ? b1 : b0) + __shfl_xor_sync(0xffffffffu, u4 ? b0 : b1, 4);
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  c += __shfl_xor_sync(0xffffffffu, c, 1);
+  return c;
+}
+__device__ __forceinline__ int warp_slot() {  // lanes 0, 8, 4, 16, 24 hold v[0] .. v[4]
+  const int lane = threadIdx.x & 31;
+  return (lane & 3) != 0 || ((lane & 4) && lane != 4) ? -1 : lane & 4 ? 2 : (lane >> 4) * 3 + (lane >> 3 & 1);
+}
+
+// The block's sum of v[q], returned to thread q < 5; fixed order.  sh is free again after the
+// block's next barrier.
 template <int NT>
-__device__ __forceinline__ double block_sum5(double* v, double* sh) {
-  // v[5] per thread -> sh[0..4] in thread 0; fixed tree order
-#pragma unroll
-  for (int q = 0; q < 5; ++q) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-  }
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0)
-#pragma unroll
-    for (int q = 0; q < 5; ++q) sh[w * 5 + q] = v[q];
+__device__ __forceinline__ double block_sum5(const double* v, double* sh) {
+  const double c = warp_sum5(v);
+  const int slot = warp_slot();
+  if (slot >= 0) sh[(threadIdx.x >> 5) * 5 + slot] = c;
   __syncthreads();
-  if (threadIdx.x < 32) {
+  double t = 0.0;
+  if (threadIdx.x < 5)
 #pragma unroll
-    for (int q = 0; q < 5; ++q) {
-      double t = threadIdx.x < NT / 32 ? sh[threadIdx.x * 5 + q] : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-      v[q] = t;
-    }
-  }
-  __syncthreads();
-  return v[0];
+    for (int i = 0; i < NT / 32; ++i) t += sh[i * 5 + threadIdx.x];
+  return t;
 }
 
 // Per pixel: I = q2 (Fr Sa Sb)^2 and its derivatives
@@ -361,10 +415,9 @@ __global__ void __launch_bounds__(NT) cyl_pixels_kernel(CylArgs a) {
       }
     }
     if (a.counts) {
-      block_sum5<NT>(acc, sh);
-      if (threadIdx.x == 0)
-#pragma unroll
-        for (int q = 0; q < 5; ++q) a.partial[5 * it + q] = acc[q];
+      const double t = block_sum5<NT>(acc, sh);
+      if (threadIdx.x < 5) a.partial[5 * it + threadIdx.x] = t;
+      __syncthreads();
     }
   }
 }
@@ -378,104 +431,121 @@ __global__ void __launch_bounds__(NT) cyl_pixels_kernel(CylArgs a) {
 // both signs over the detector, and such an error would add up where the residuals cancel.
 // Row and column advance by integer steps (no division per pixel); weights w come from a
 // per-pixel FP32 array made once when the batch is created.
+// An item is what one warp does between two sums: 32 lanes x per_lane pixels in a row of the region,
+// per_lane by the region's size alone (cyl_apply_shape), so that a candidate's result does not
+// depend on its company.  Warps share nothing and meet at no barrier.  48 regions of 96 to 640 pixels
+// a side: 106 us; with items of a block of 256 (a block sum, a load of the candidate and barriers for every
+// 1,024 pixels) 110, with the candidate's fields, the 4-point weights and the Dirichlet kernels
+// loaded and computed singly as well 128.  Bound by issue (340 instructions a pixel, 12 of them
+// conversions between FP32 and FP64) and the latency of two dependent loads; the 12 bytes per
+// pixel would take 12 us.
 template <int NT, int PPT>
 __global__ void __launch_bounds__(NT) cyl_pixels_f32c_kernel(CylArgs a) {
-  __shared__ double sh[(NT / 32) * 5];
-  for (long it = blockIdx.x; it < a.nitems; it += gridDim.x) {
-    const int2 item = a.items[it];
-    const CylCand& c = a.cands[item.x];
-    const int ncols = c.ncols;
-    const long npx = (long)c.nrows * ncols;
-    const int first = item.y + threadIdx.x;
-    int lr = first / ncols, lc = first - lr * ncols;
-    const int dq = NT / ncols, dr = NT - dq * ncols;
+  constexpr int W = NT / 32;
+  __shared__ CylPix s_k[W];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slot = warp_slot();
+  for (long it = (long)blockIdx.x * W + warp; it < a.nitems; it += (long)gridDim.x * W) {
+    const int2 item = __ldg(a.items + it);
+    __syncwarp();  // s_k is read no more
+    if (lane < (int)(sizeof(CylPix) / 16))
+      reinterpret_cast<uint4*>(&s_k[warp])[lane] =
+          __ldg(reinterpret_cast<const uint4*>(&a.cands[item.x].pix) + lane);
+    __syncwarp();
+    const CylPix& k = s_k[warp];
+    const int ncols = k.ncols;
+    const int last = min((int)((long)k.nrows * ncols), item.y + 32 * k.per_lane);
+    int idx = item.y + lane;
+    int lr = idx / ncols, lc = idx - lr * ncols;
+    const RowTab* tab = a.tab + k.rowtab0;
+    const CylCell* table = a.table + (long)item.x * CYL_NTAB;
+    const long px_off = k.px_off;
     float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < PPT; ++j) {
-      if (j > 0) {
-        lr += dq;
-        lc += dr;
-        if (lc >= ncols) {
-          lc -= ncols;
-          ++lr;
+      if (idx < last) {
+        const long p = (long)(k.row0 + lr) * a.grid_ncol + (k.col0 + lc);
+        const double qx = __ldg(a.qx + p), qy = __ldg(a.qy + p);
+        // the pixel's counts and weight issued early (read-only loads, independent of the math)
+        double C = 0.0;
+        float w = 0.0f;
+        if (a.counts) {
+          C = __ldg(a.counts + px_off + idx);
+          w = __ldg(a.wf + px_off + idx);
         }
-      }
-      const long idx = (long)first + (long)j * NT;
-      if (idx >= npx) continue;
-      const long p = (long)(c.row0 + lr) * a.grid_ncol + (c.col0 + lc);
-      const double qx = __ldg(a.qx + p), qy = __ldg(a.qy + p);
-      // the pixel's counts and weight issued early (read-only loads, independent of the math)
-      double C = 0.0;
-      float w = 0.0f;
-      if (a.counts) {
-        C = __ldg(a.counts + c.px_off + idx);
-        w = __ldg(a.wf + c.px_off + idx);
-      }
-      const double mx = c.cphi * qx - c.sphi * qy, my = c.sphi * qx + c.cphi * qy;
-      const double q2d = mx * mx + my * my;
-      float FR = 0.f, FRR = 0.f;
-      if (q2d * c.rmin * c.rmin > 1.0e-13) {
-        // node below u = q_par / h + 1 by the FP64 rounding constant (its low word is the index)
-        const double u = sqrt(q2d) * a.inv_h + 1.0;
-        const double rb = __dadd_rn(__dadd_rn(u, -0.5), RND52);
-        const int k = __double2loint(rb), i0 = min(max(k, 1), CYL_NTAB - 3);
-        float t = (float)(u - __dsub_rn(rb, RND52));
-        if (i0 != k) t += (float)(k - i0);
-        const float w0 = -t * (t - 1.0f) * (t - 2.0f) * (1.0f / 6.0f);
-        const float w1 = (t + 1.0f) * (t - 1.0f) * (t - 2.0f) * 0.5f;
-        const float w2 = -(t + 1.0f) * t * (t - 2.0f) * 0.5f;
-        const float w3 = (t + 1.0f) * t * (t - 1.0f) * (1.0f / 6.0f);
-        const float4* tb = a.table + (long)item.x * CYL_NTAB + (i0 - 1);
-        const float4 f0 = __ldg(tb), f1 = __ldg(tb + 1), f2 = __ldg(tb + 2), f3 = __ldg(tb + 3);
-        FR = (w0 * f0.x + w1 * f1.x + w2 * f2.x + w3 * f3.x) + (w0 * f0.y + w1 * f1.y + w2 * f2.y + w3 * f3.y);
-        FRR = (w0 * f0.z + w1 * f1.z + w2 * f2.z + w3 * f3.z) + (w0 * f0.w + w1 * f1.w + w2 * f2.w + w3 * f3.w);
-      } else {  // the reference's q_par -> 0 guard: sum the terms that pass it
-        const float qp = (float)sqrt(q2d);
-        for (int i = 0; i < c.nr; ++i) {
-          const float r = (float)c.r[i], x = qp * r;
-          if ((double)x * (double)x > 1.0e-13) {
-            const float two_pi_r = (float)(2.0 * PI_D) * r;
-            FR += two_pi_r * r * j1f(x) / x;
-            FRR += two_pi_r * r * j0f(x);
+        const double mx = k.cphi * qx - k.sphi * qy, my = k.sphi * qx + k.cphi * qy;
+        const double q2d = mx * mx + my * my;
+        float FR = 0.f, FRR = 0.f;
+        if (q2d > k.qmin2) {
+          // sqrt(q2d) by one Newton step from the FP32 reciprocal root (e below 1e-6: 3/8 e^2 is left)
+          const double y = (double)rsqrtf(fmaxf((float)q2d, 1e-37f)), s = q2d * y, e = fma(-s, y, 1.0);
+          // interval below u = q_par / h + 1 by the FP64 rounding constant (its low word is the index)
+          const double u = fma(fma(0.5 * s, e, s), a.inv_h, 1.0);
+          const double rb = __dadd_rn(__dadd_rn(u, -0.5), RND52);
+          const int iu = __double2loint(rb), i0 = min(max(iu, 1), CYL_NTAB - 3);
+          float t = (float)(u - __dsub_rn(rb, RND52));
+          if (i0 != iu) t += (float)(iu - i0);
+          const CylCell* cell = table + i0;
+          const float4 f = __ldg(&cell->fr), g = __ldg(&cell->frR);
+          const float2 lo = __ldg(&cell->lo);
+          FR = f.x + (lo.x + t * (f.y + t * (f.z + t * f.w)));
+          FRR = g.x + (lo.y + t * (g.y + t * (g.z + t * g.w)));
+        } else {  // the reference's q_par -> 0 guard: sum the terms that pass it
+          const float qp = (float)sqrt(q2d);
+          const CylCand& c = a.cands[item.x];
+          for (int i = 0; i < c.nr; ++i) {
+            const float r = (float)c.r[i], x = qp * r;
+            if ((double)x * (double)x > 1.0e-13) {
+              const float two_pi_r = (float)(2.0 * PI_D) * r;
+              FR += two_pi_r * r * j1f(x) / x;
+              FRR += two_pi_r * r * j0f(x);
+            }
           }
+          FRR /= (float)c.R;
         }
-        FRR /= (float)c.R;
+        double ta = k.ka[0] * mx + k.ka[1] * my, tb = k.kb[0] * mx + k.kb[1] * my;
+        ta -= round_fp64(ta);
+        tb -= round_fp64(tb);
+        float2 S2, dS2;
+        dirichlet_pair(ta, tb, k, &S2, &dS2);
+        const float Sa = S2.x, Sb = S2.y;
+        const float4 rt = __ldg(reinterpret_cast<const float4*>(tab + lr));  // q2, q2f, qhf
+        const double q2 = __hiloint2double(__float_as_int(rt.y), __float_as_int(rt.x));
+        const float SS = Sa * Sb, F = FR * SS;
+        const double I = q2 * (double)(F * F);
+        if (a.intensity) a.intensity[px_off + idx] = I;
+        if (a.counts) {
+          const float X = (float)mx, Y = (float)my;
+          const float2 X2 = make_float2(X, X), Y2 = make_float2(Y, Y), v0 = make_float2(k.fu0[0], k.fu0[1]),
+                       v1 = make_float2(k.fu1[0], k.fu1[1]), D = __fmul2_rn(dS2, make_float2(Sb, Sa));
+          const float2 pa = __fmul2_rn(D, __ffma2_rn(v0, X2, __fmul2_rn(v1, Y2)));
+          const float2 ra = __fmul2_rn(D, __ffma2_rn(v1, X2, __fmul2_rn(v0, make_float2(-Y, -Y))));
+          const float dSSa = pa.x + pa.y;
+          const float dSSp = k.fa * (ra.x + ra.y);
+          const float FRF = FR * F;
+          const float q2f = rt.z, qhf = rt.w, qaf = __ldg(&tab[lr].qaf);
+          const float res = (float)(k.scale * I - C);
+          const float g = 2.0f * w * res * k.fscale;
+          acc[0] += w * res * res;
+          acc[1] += g * (2.0f * q2f * F * FRR * SS);
+          acc[2] += g * (2.0f * qhf * F * F);
+          acc[3] += g * (2.0f * FRF * (q2f * dSSa + qaf * SS));
+          acc[4] += g * (2.0f * q2f * FRF * dSSp);
+        }
       }
-      double ta = c.ka[0] * mx + c.ka[1] * my, tb = c.kb[0] * mx + c.kb[1] * my;
-      ta -= round_fp64(ta);
-      tb -= round_fp64(tb);
-      float Sa, dSa, Sb, dSb;
-      dirichlet_f32(ta, c.rep[0], c.frep[0], c.ser[0], &Sa, &dSa);
-      dirichlet_f32(tb, c.rep[1], c.frep[1], c.ser[1], &Sb, &dSb);
-      const RowTab* rt = a.tab + c.rowtab0 + lr;
-      const float SS = Sa * Sb, F = FR * SS;
-      const double I = __ldg(&rt->q2) * (double)(F * F);
-      if (a.intensity) a.intensity[c.px_off + idx] = I;
-      if (a.counts) {
-        const float X = (float)mx, Y = (float)my;
-        const float pa = c.fua[0] * X + c.fua[1] * Y, pb = c.fub[0] * X + c.fub[1] * Y;
-        const float ra = c.fua[1] * X - c.fua[0] * Y, rb = c.fub[1] * X - c.fub[0] * Y;
-        const float dSSa = dSa * pa * Sb + Sa * dSb * pb;
-        const float dSSp = c.fa * (dSa * ra * Sb + Sa * dSb * rb);
-        const float FRF = FR * F;
-        const float q2f = __ldg(&rt->q2f), qhf = __ldg(&rt->qhf), qaf = __ldg(&rt->qaf);
-        const float res = (float)(c.scale * I - C);
-        const float g = 2.0f * w * res * c.fscale;
-        acc[0] += w * res * res;
-        acc[1] += g * (2.0f * q2f * F * FRR * SS);
-        acc[2] += g * (2.0f * qhf * F * F);
-        acc[3] += g * (2.0f * FRF * (q2f * dSSa + qaf * SS));
-        acc[4] += g * (2.0f * q2f * FRF * dSSp);
+      idx += 32;
+      lr += k.dq;
+      lc += k.dr;
+      if (lc >= ncols) {
+        lc -= ncols;
+        ++lr;
       }
     }
     if (a.counts) {
-      double accd[5];
+      double sum[5];
 #pragma unroll
-      for (int q = 0; q < 5; ++q) accd[q] = (double)acc[q];
-      block_sum5<NT>(accd, sh);
-      if (threadIdx.x == 0)
-#pragma unroll
-        for (int q = 0; q < 5; ++q) a.partial[5 * it + q] = accd[q];
+      for (int q = 0; q < 5; ++q) sum[q] = (double)acc[q];
+      const double t = warp_sum5(sum);
+      if (slot >= 0) a.partial[5 * it + slot] = t;
     }
   }
 }
@@ -501,15 +571,12 @@ __global__ void cyl_final_kernel(const CylCand* __restrict__ cands, const double
   for (long i = threadIdx.x; i < c.nitems; i += CYL_THREADS)
 #pragma unroll
     for (int q = 0; q < 5; ++q) acc[q] += partial[5 * (c.item0 + i) + q];
-  block_sum5<CYL_THREADS>(acc, sh);
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < 5; ++q) out[5 * blockIdx.x + q] = acc[q];
-    if (blockIdx.x == 0) {
-      double e = 0.0;
-      *reinterpret_cast<unsigned*>(&e) = *err;
-      out[5 * ncand] = e;
-    }
+  const double t = block_sum5<CYL_THREADS>(acc, sh);
+  if (threadIdx.x < 5) out[5 * blockIdx.x + threadIdx.x] = t;
+  if (threadIdx.x == 0 && blockIdx.x == 0) {
+    double e = 0.0;
+    *reinterpret_cast<unsigned*>(&e) = *err;
+    out[5 * ncand] = e;
   }
 }
 
@@ -602,7 +669,7 @@ __global__ void __launch_bounds__(128) cyl_plain_kernel(const CylCand* __restric
 }
 
 // ------------------------------------------------------------------- host ----
-// Scaled power sums of the FP32C Dirichlet series (dirichlet_f32): with c_j = j - (N-1)/2,
+// Scaled power sums of the FP32C Dirichlet series (dirichlet_pair): with c_j = j - (N-1)/2,
 // s_2k = sum_j c_j^2k (polynomials in N, exact for integer N: N(N^2-1)/12,
 // N(N^2-1)(3N^2-7)/240, N(N^2-1)(3N^4-18N^2+31)/1344, N(N^2-1)(5N^6-55N^4+239N^2-381)/11520),
 //   S  = N (1 - y e0 + y^2 e1 - y^3 e2 + y^4 e3),          e_k = s_2k+2 / ((2k+2)! N^(2k+3)),
@@ -646,14 +713,20 @@ int cyl_fill_cand(const double* m, const double* abc9, const int* roi, double sc
   c.ub[0] = abc9[3];
   c.ub[1] = abc9[4];
   c.uc = abc9[8];
-  c.fa = (float)c.a;
+  c.pix.cphi = c.cphi;
+  c.pix.sphi = c.sphi;
+  c.pix.fa = (float)c.a;
+  c.pix.fu0[0] = (float)c.ua[0];
+  c.pix.fu0[1] = (float)c.ub[0];
+  c.pix.fu1[0] = (float)c.ua[1];
+  c.pix.fu1[1] = (float)c.ub[1];
   for (int i = 0; i < 2; ++i) {
-    c.ka[i] = c.a * c.ua[i] / (2.0 * PI_D);
-    c.kb[i] = c.a * c.ub[i] / (2.0 * PI_D);
-    c.fua[i] = (float)c.ua[i];
-    c.fub[i] = (float)c.ub[i];
-    c.frep[i] = (float)c.rep[i];
-    cyl_dirichlet_series(c.rep[i], c.ser[i]);
+    c.pix.ka[i] = c.a * c.ua[i] / (2.0 * PI_D);
+    c.pix.kb[i] = c.a * c.ub[i] / (2.0 * PI_D);
+    c.pix.rep[i] = c.rep[i];
+    c.pix.frep[i] = (float)c.rep[i];
+    cyl_dirichlet_series(c.rep[i], c.pix.ser[i]);
+    c.pix.lim[i] = c.rep[i] == 1.0 ? INFINITY : 1.0f;
   }
   // size distributions: Gaussian over +-3 sigma sampled as param_distribution does
   double s = m[M_SPREAD];
@@ -679,14 +752,16 @@ int cyl_fill_cand(const double* m, const double* abc9, const int* roi, double sc
   c.nr = (int)rv.size();
   c.nh = (int)hv.size();
   for (int i = 0; i < c.nr; ++i) c.r[i] = rv[i];
-  c.rmin = c.nr > 0 ? *std::min_element(rv.begin(), rv.end()) : 0.0;
+  const double rmin = rv.empty() ? 0.0 : *std::min_element(rv.begin(), rv.end());
+  c.pix.qmin2 = 1.0e-13 / (rmin * rmin);
   for (int i = 0; i < c.nh; ++i) c.h[i] = hv[i];
   c.row0 = roi[0];
   c.col0 = roi[1];
   c.nrows = roi[2];
   c.ncols = roi[3];
   c.scale = scale;
-  c.fscale = (float)scale;
+  c.pix.scale = scale;
+  c.pix.fscale = (float)scale;
   return HGX_OK;
 }
 
@@ -698,7 +773,9 @@ struct hgx_cyl_batch_s {
   hgx_ctx ctx = nullptr;
   hgx_qgrid grid = nullptr;
   int ncand = 0;
-  long npx = 0, nitems = 0, nrowtab = 0;
+  long npx = 0, nrowtab = 0;
+  long nitems = 0;      // tiles of the shape
+  long nitems_dev = 0;  // entries of d_items: the tiles, or the warps' items of FP32C
   int precision = HGX_F32C;
   double abc9[9];
   std::vector<int> rois;
@@ -724,17 +801,16 @@ static int cyl_enqueue(hgx_cyl_batch_s* b, bool with_counts, bool with_intensity
                            cudaMemcpyHostToDevice, st));
   int maxrows = 0;
   for (int i = 0; i < b->ncand; ++i) maxrows = std::max(maxrows, b->rois[4 * i + 2]);
-  // row table (a warp per row, 4 rows per block) and, in FP32C, the radial-sum tables (16
-  // nodes per block) in one launch
-  const int row_blocks = (maxrows + 3) / 4;
-  const int table_blocks = b->precision == HGX_F32C ? (8 * CYL_NTAB + 127) / 128 : 0;
-  cyl_prep_kernel<<<dim3(row_blocks + table_blocks, b->ncand), 128, 0, st>>>(
+  // row table (a warp per row) and, in FP32C, the radial-sum tables
+  // (CYL_CELLS intervals per block, the last one CYL_NTAB - 3) in one launch
+  const int row_blocks = (maxrows + CYL_PREP_THREADS / 32 - 1) / (CYL_PREP_THREADS / 32);
+  const int table_blocks = b->precision == HGX_F32C ? (CYL_NTAB - 3 + CYL_CELLS - 1) / CYL_CELLS : 0;
+  cyl_prep_kernel<<<dim3(row_blocks + table_blocks, b->ncand), CYL_PREP_THREADS, 0, st>>>(
       (const CylCand*)b->d_cands.p, row_blocks, b->grid->rowqz, (const double2*)b->d_rowfc.p,
-      (RowTab*)b->d_tab.p, b->table_h, (float4*)b->d_table.p);
+      (RowTab*)b->d_tab.p, b->table_h, (CylCell*)b->d_table.p);
   CylArgs a;
   a.cands = (const CylCand*)b->d_cands.p;
   a.items = (const int2*)b->d_items.p;
-  a.nitems = b->nitems;
   a.tab = (const RowTab*)b->d_tab.p;
   a.qx = b->grid->qx;
   a.qy = b->grid->qy;
@@ -743,10 +819,12 @@ static int cyl_enqueue(hgx_cyl_batch_s* b, bool with_counts, bool with_intensity
   a.mask = with_counts ? (const unsigned*)b->d_mask.p : nullptr;
   a.intensity = with_intensity ? (double*)b->d_inten.p : nullptr;
   a.partial = (double*)b->d_partial.p;
-  a.table = (const float4*)b->d_table.p;
+  a.table = (const CylCell*)b->d_table.p;
   a.inv_h = 1.0 / b->table_h;
   a.wf = with_counts ? (const float*)b->d_wf.p : nullptr;
-  long blocks = std::min<long>(b->nitems, (long)b->persistent_blocks);
+  a.nitems = b->nitems_dev;
+  const int per_block = b->precision == HGX_F64 ? 1 : CYL_SHAPES[b->shape].threads / 32;
+  const long blocks = std::min<long>((b->nitems_dev + per_block - 1) / per_block, (long)b->persistent_blocks);
   cudaError_t e = b->precision == HGX_F64
                       ? cyl_pixels_at<double, 0>(b->shape, (unsigned)blocks, a, st, nullptr)
                       : cyl_pixels_at<float, 0>(b->shape, (unsigned)blocks, a, st, nullptr);
@@ -773,12 +851,21 @@ static int cyl_apply_shape(hgx_cyl_batch_s* b, int shape) {
     return fail(HGX_ERR_INVALID_ARG, "hgx_cyl_batch: unknown tile shape");
   const long tile = (long)CYL_SHAPES[shape].threads * CYL_SHAPES[shape].ppt;
   std::vector<int2> items;
+  long tiles = 0;
   for (int i = 0; i < b->ncand; ++i) {
     CylCand& h = b->h_cands[i];
-    long n = (long)b->rois[4 * i + 2] * b->rois[4 * i + 3];
+    const int ncols = b->rois[4 * i + 3];
+    const long n = (long)b->rois[4 * i + 2] * ncols;
+    // FP32C: a warp's items, one pixel per lane in regions below 2^16 pixels (which then spread over
+    // more warps) up to the shape's number from 2^15 pixels each on
+    h.pix.per_lane = (int)std::max<long>(1, std::min<long>(CYL_SHAPES[shape].ppt, n >> 15));
+    h.pix.dq = 32 / ncols;
+    h.pix.dr = 32 % ncols;
+    const long step = b->precision == HGX_F64 ? tile : 32L * h.pix.per_lane;
     h.item0 = (long)items.size();
-    for (long s = 0; s < n; s += tile) items.push_back(make_int2(i, (int)s));
+    for (long s = 0; s < n; s += step) items.push_back(make_int2(i, (int)s));
     h.nitems = (long)items.size() - h.item0;
+    tiles += (n + tile - 1) / tile;
   }
   cudaStream_t st = b->ctx->stream;
   HGX_CUDA(cudaStreamSynchronize(st));
@@ -797,7 +884,8 @@ static int cyl_apply_shape(hgx_cyl_batch_s* b, int shape) {
                                           : cyl_pixels_at<float, 0>(shape, 0, none, st, &per_sm);
   if (e != cudaSuccess) return cuda_fail(e, "hgx_cyl_batch: occupancy query");
   b->persistent_blocks = b->ctx->sm_count * std::max(1, per_sm);
-  b->nitems = (long)items.size();
+  b->nitems = tiles;
+  b->nitems_dev = (long)items.size();
   b->shape = shape;
   return HGX_OK;
 }
@@ -812,6 +900,15 @@ static int cyl_set_models(hgx_cyl_batch_s* b, const double* models) {
     c.item0 = h.item0;
     c.nitems = h.nitems;
     c.rowtab0 = h.rowtab0;
+    c.pix.per_lane = h.pix.per_lane;
+    c.pix.dq = h.pix.dq;
+    c.pix.dr = h.pix.dr;
+    c.pix.px_off = c.px_off;
+    c.pix.rowtab0 = c.rowtab0;
+    c.pix.row0 = c.row0;
+    c.pix.col0 = c.col0;
+    c.pix.nrows = c.nrows;
+    c.pix.ncols = c.ncols;
     h = c;
   }
   return HGX_OK;
@@ -902,7 +999,7 @@ int hgx_cyl_batch_create(hgx_ctx c, hgx_qgrid g, const double* rowfc, const doub
     double qm = 0.0;
     for (int i = 0; i < g->nqy; ++i) qm = std::max(qm, sqrt(hx[i] * hx[i] + hy[i] * hy[i]));
     b->table_h = (qm > 0.0 ? qm : 1.0) * (1.0 + 1e-9) / CYL_QT;
-    if ((s = b->d_table.reserve(sizeof(float4) * CYL_NTAB * (size_t)ncand))) return bail(s);
+    if ((s = b->d_table.reserve(sizeof(CylCell) * CYL_NTAB * (size_t)ncand))) return bail(s);
     if (counts) {
       if ((s = b->d_wf.reserve(sizeof(float) * px))) return bail(s);
       cyl_weights_kernel<<<(unsigned)std::min<long>((px + 255) / 256, 4L * c->sm_count * 8), 256, 0, st>>>(

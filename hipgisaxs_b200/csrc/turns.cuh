@@ -41,6 +41,31 @@ __device__ __forceinline__ void sincospi_f32(float x, float* s, float* c) {
   *c = co;
 }
 
+// The same for two numbers, two to an FP32x2 operation.
+__device__ __forceinline__ void sincospi_f32x2(float2 x, float2* s, float2* c) {
+  auto two = [](float v) { return make_float2(v, v); };
+  const float2 b = __ffma2_rn(two(2.0f), x, two(12582912.0f));
+  const float2 r = __ffma2_rn(two(-0.5f), __fadd2_rn(b, two(-12582912.0f)), x), r2 = __fmul2_rn(r, r);
+  float2 ps = __ffma2_rn(two(0.08214588463306427f), r2, two(-0.5992645025253296f));
+  ps = __ffma2_rn(ps, r2, two(2.550163984298706f));
+  ps = __ffma2_rn(ps, r2, two(-5.167712688446045f));
+  ps = __ffma2_rn(ps, r2, two(3.1415927410125732f));
+  float2 pc = __ffma2_rn(two(-0.025806890800595284f), r2, two(0.23533062636852264f));
+  pc = __ffma2_rn(pc, r2, two(-1.3352627754211426f));
+  pc = __ffma2_rn(pc, r2, two(4.058712005615234f));
+  pc = __ffma2_rn(pc, r2, two(-4.934802055358887f));
+  pc = __ffma2_rn(pc, r2, two(1.0f));
+  const float2 sv = __fmul2_rn(r, ps);
+  // quarter q: sin takes its sign from bit 1 of q, cos from bit 1 of q + 1
+  auto turn = [](float bq, float sn, float cs, float* so, float* co) {
+    const unsigned q = __float_as_uint(bq);
+    *so = __uint_as_float(__float_as_uint(q & 1 ? cs : sn) ^ ((q & 2) << 30));
+    *co = __uint_as_float(__float_as_uint(q & 1 ? sn : cs) ^ (((q + 1) & 2) << 30));
+  };
+  turn(b.x, sv.x, pc.x, &s->x, &c->x);
+  turn(b.y, sv.y, pc.y, &s->y, &c->y);
+}
+
 // sin(pi x) for |x| <= 1/2 in FP32: x times a polynomial of degree 4 in x^2 (a Chebyshev fit;
 // within 1.5e-7 of the value, relative near 0, 3.6e-8 rms).
 __device__ __forceinline__ float sin_half_turn(float x) {

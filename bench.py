@@ -35,46 +35,47 @@ NCOL = NROW = 2048
 QMIN_Y, QMIN_Z, QMAX_Y, QMAX_Z = -2.0, 0.0, 2.0, 3.0
 ENERGY_KEV, ALPHA_I_DEG = 10.0, 0.20
 PI_REF = 3.141592653589793
-# FP32 FLOP of the row-factorised kernel per (pixel, triangle) for the 4 paired real
-# DWBA blocks (FMA = 2): in-plane phase offset q_par.d 3, in-plane q_par.n~ 3, U = (q.n~) E 2,
-# 16 FFMA accumulations 32 -> 40 FLOP and 2 SFU ops (sin, cos) per 4 evaluations.  Not
-# counted: the explicit reduction on wide tiles, the per-tile anchor rotation and TwoSum fold.
+# The row kernel per (pixel, triangle) with the 4 paired real DWBA blocks: 2 SFU operations
+# (sin, cos of the in-plane phase) and, on the tensor cores, 192 int8 products (3 digits of each x
+# 96 columns of row-factor digits).  The factorised sum written with FP32 operations (FMA = 2): phase 3, q_par.n~ 3, U 2,
+# 16 accumulating FMA 32 -> 40 FLOP.
 FLOP_PER_PIXEL_TRI = 40.0
 SFU_PER_PIXEL_TRI = 2.0
-# DRAM bytes per launch of the row kernel: ncu dram__bytes_read.sum + dram__bytes_write.sum
-# of one 2048 x 2048 launch with 50,000 triangles (75.2 MB read + 84.8 MB written)
-TRAFFIC_BYTES_PER_LAUNCH = 160.0e6
-TRAFFIC_SOURCE = "ncu capture of a 2048x2048 launch (75.2 MB read + 84.8 MB write)"
-# the library's kernels per form-factor step (bounding box 2, Morton keys, tiles, row kernel);
+INT8_OPS_PER_PIXEL_TRI = 384.0
+# DRAM bytes per step: the row factors' digits (2048 rows x 98 tiles x 24,640 bytes) written and
+# read once, the q-grid and the output.  At 512 x 512 x 20,000 ncu counts 444 MB written and 510 MB
+# read for 504 MB of digits.
+TRAFFIC_BYTES_PER_LAUNCH = 2 * 4.95e9 + 201.0e6
+TRAFFIC_SOURCE = "row-factor digits 2 x 4.95 GB (by layout; ncu at 512x512 agrees), q-grid and output"
+# the library's kernels per form-factor step (bounding box 2, Morton keys, tiles, and for each of
+# five slabs of row factors their kernel and the row kernel);
 # CUB's radix sort of the keys adds 6 launches per step
-HGX_LAUNCHES_PER_STEP = 5
+HGX_LAUNCHES_PER_STEP = 14
 CUB_LAUNCHES_PER_STEP = 6
 
 
 # Executed FLOP per unit of the other timed kernels, from ncu thread-instruction counts
 # (2 x FMA + MUL + ADD of each precision) of one launch on the bench's own descriptions,
 # each from an ncu capture of its kernel on the workload below:
-#   mesh_backward_kernel     82.5 FP32 per (pixel, triangle)   (the expression: 80)
+#   (the mesh vertex gradient is held against the SFU: 2 operations per pass and (pixel, triangle))
 #   ff_exact_kernel          611 FP64 per (q-point, triangle)
-#   grain_dwba_kernel        6418 FP64 per (pixel, grain), hcp cylinders (HIG_ENSEMBLE)
-#   grain_dwba_f32c_kernel   1060 FP32 + 408 FP64 per (pixel, grain), the same description
-#   cyl_pixels_f32c_kernel   221 FP32 + 60 FP64 per ROI pixel (the 256-candidate batch)
+#   grain_dwba_real_kernel<double>  363 FP64 per (pixel, grain), hcp cylinders (HIG_ENSEMBLE)
+#   grain_dwba_real_kernel<float>   147 FP32 + 68 FP64 per (pixel, grain), the same description
+#   cyl_pixels_f32c_kernel   200 FP32 + 52 FP64 per ROI pixel (FP32x2 counted as two)
 #   cyl_pixels_kernel<double>  1418 FP64 per ROI pixel (the same batch)
-#   grain_dwba_f32c_kernel   1340 FP32 + 554 FP64 and 159 XU-pipe operations per pixel (config 1)
-#   grain_dwba_kernel        16999 FP64 per pixel (config 1)
-CYL_F32C_FP32_FLOP_PER_PIXEL = 221.0
-CYL_F32C_FP64_FLOP_PER_PIXEL = 60.0
+#   grain_dwba_real_kernel<float>   978 FP32 + 307 FP64 and 118 XU-pipe operations per pixel (config 1)
+#   grain_dwba_real_kernel<double>  1414 FP64 per pixel (config 1)
+CYL_F32C_FP32_FLOP_PER_PIXEL = 200.0
+CYL_F32C_FP64_FLOP_PER_PIXEL = 52.0
 CYL_F64_FLOP_PER_PIXEL = 1418.0
-CFG1_F32C_FP32_FLOP_PER_PIXEL = 1340.0
-CFG1_F32C_FP64_FLOP_PER_PIXEL = 554.0
-CFG1_F32C_XU_PER_PIXEL = 159.0
-CFG1_F64_FLOP_PER_PIXEL = 16999.0
-MESH_FWD_FLOP_PER_PIXEL_TRI = FLOP_PER_PIXEL_TRI
-MESH_BWD_FLOP_PER_PIXEL_TRI = 80.0
+CFG1_F32C_FP32_FLOP_PER_PIXEL = 978.0
+CFG1_F32C_FP64_FLOP_PER_PIXEL = 307.0
+CFG1_F32C_XU_PER_PIXEL = 118.0
+CFG1_F64_FLOP_PER_PIXEL = 1414.0
 EXACT_FP64_FLOP_PER_EVAL = 611.0
-GRAIN_FP64_FLOP_PER_PIXEL_GRAIN = 6418.0
-GRAIN_F32C_FP32_FLOP_PER_PIXEL_GRAIN = 1060.0
-GRAIN_F32C_FP64_FLOP_PER_PIXEL_GRAIN = 408.0
+GRAIN_FP64_FLOP_PER_PIXEL_GRAIN = 363.0
+GRAIN_F32C_FP32_FLOP_PER_PIXEL_GRAIN = 147.0
+GRAIN_F32C_FP64_FLOP_PER_PIXEL_GRAIN = 68.0
 
 
 def roofline_of(bound, flop_per_unit, units, seconds, peak, unit, source):
@@ -141,7 +142,7 @@ def parse():
                     help="detector rows = columns of the form-factor workload (default 2048; "
                          "smaller grids are for profiling captures, not bench lines)")
     ap.add_argument("--ppt", type=int, default=0,
-                    help="row-kernel pixels per thread (0: the library's autotuner chooses)")
+                    help="launch shape of the FP32 row kernel (0: the library's automatic kernel)")
     return ap.parse_args()
 
 
@@ -648,9 +649,9 @@ def config1_bench(ctx, steps=3, n=1024, cpu=True, dev_steps=20):
     i32, i64 = imgs["f32c"].ravel(), imgs["f64"].ravel()
     res["value"] = res["f32c"]["value"]
     res["fp32c_speedup_vs_fp64"] = res["f64"]["ms"] / res["f32c"]["ms"]
-    res["fp32c_vs_fp64_note"] = ("beside FP32 arithmetic the FP32C grain kernel sums the cylinder heights in "
-                                 "closed form; the FP64 kernel keeps the reference's per-sample height sums "
-                                 "(1e-11 parity); both share the in-plane sums across a pixel's four lanes")
+    res["fp32c_vs_fp64_note"] = ("the same kernel: FP32C forms and reduces the phases in FP64 and takes the "
+                                 "transcendentals and sums in FP32; both make the in-plane sums once for a "
+                                 "pixel's four blocks and sum evenly stepped heights in closed form")
     res["timing"] = (f"device image: {dev_steps} back-to-back calls between CUDA events on the launching "
                      "stream (each call returns once queued: tables, grain kernel, structure sum); "
                      "e2e_ms_host_image: one synchronous call with the 8 MB image copied to pageable "
@@ -803,16 +804,9 @@ def main():
     sd_dev = torch.tensor(sd, device=dev)
     out = torch.empty(4 * n, dtype=torch.complex64, device=dev)
 
-    # launch shape chosen by the library's autotuner on this grid (outside the timed region;
-    # 8,192 triangles rank the candidates, whose cost is linear in the triangle count)
-    if args.ppt:
-        tuned_p, tune_times = args.ppt, {}
-    else:
-        tuned_p, _, tune_times = hg.ff_tune(ctx, grid, sd_dev[:8192], None, "c64", reps=2)
-
     def step():
         hg.ff_triangles(ctx, grid, sd_dev, None, "f32c", out=out, out_type="c64",
-                        pixels_per_thread=tuned_p)
+                        pixels_per_thread=args.ppt)
 
     def barrier():
         if dist is not None:
@@ -910,17 +904,17 @@ def main():
         bt = fit["batch_256_rois"]
         bt["roofline"] = roofline_of(
             "fp32", CYL_F32C_FP32_FLOP_PER_PIXEL, float(bt["pixels"]), bt["ms_per_batch"] * 1e-3, peak_fp32,
-            "ROI pixel", "ncu executed FP32 FLOP of cyl_pixels_f32c_kernel (plus 60 FP64 per pixel); issue-"
-            "bound with no pipe above 31% in ncu; the time is the whole graph (set-up, pixel pass, sums)")
+            "ROI pixel", "ncu executed FP32 FLOP of cyl_pixels_f32c_kernel (plus 52 FP64 per pixel); issue-"
+            "bound with no pipe above 36% in ncu; the time is the whole graph (set-up, pixel pass, sums)")
         bt["fp64_adjoint"]["roofline"] = roofline_of(
             "fp64", CYL_F64_FLOP_PER_PIXEL, float(bt["pixels"]), bt["fp64_adjoint"]["ms_per_batch"] * 1e-3,
             peak_fp64, "ROI pixel", "ncu executed FP64 FLOP of cyl_pixels_kernel<double>")
         fit["mesh_vertices_2048sq"] = mesh_grad_bench(ctx, grid)
         mv = fit["mesh_vertices_2048sq"]
-        mv["roofline"] = roofline_of(
-            "fp32", MESH_FWD_FLOP_PER_PIXEL_TRI + MESH_BWD_FLOP_PER_PIXEL_TRI, float(n) * mv["triangles"],
-            mv["s_per_eval"], peak_fp32, "(pixel, triangle): forward 40 + backward 80",
-            "the expressions as written; ncu counts 82.5 executed in the backward")
+        mv_sfu = 2 * SFU_PER_PIXEL_TRI * n * mv["triangles"] / mv["s_per_eval"] / 1e9
+        mv["roofline"] = {"bound": "sfu", "ops_per_unit": 2 * SFU_PER_PIXEL_TRI,
+                          "unit": "(pixel, triangle): sine and cosine, forward and backward",
+                          "achieved": mv_sfu, "peak": peak_sfu, "units_rate": "Gop/s", "frac": mv_sfu / peak_sfu}
 
     exact = None
     if not args.no_exact and world == 1:
@@ -934,13 +928,13 @@ def main():
         pg = float(hig["pixels"]) * hig["grains"]
         hig["roofline"] = roofline_of("fp64", GRAIN_FP64_FLOP_PER_PIXEL_GRAIN, pg,
                                       hig["ms_per_simulation"] * 1e-3, peak_fp64, "(pixel, grain)",
-                                      "ncu executed FP64 FLOP of grain_dwba_kernel on this description; "
+                                      "ncu executed FP64 FLOP of grain_dwba_real_kernel on this description; "
                                       "the time is the whole simulation")
         if "f32c" in hig:
             hig["f32c"]["roofline"] = roofline_of(
                 "fp32", GRAIN_F32C_FP32_FLOP_PER_PIXEL_GRAIN, pg, hig["f32c"]["ms_per_simulation"] * 1e-3,
-                peak_fp32, "(pixel, grain)", "ncu executed FP32 FLOP of grain_dwba_f32c_kernel (plus 367 "
-                "FP64 per unit); issue-bound (80% in ncu; XU 26%)")
+                peak_fp32, "(pixel, grain)", "ncu executed FP32 FLOP of grain_dwba_real_kernel (plus 68 "
+                "FP64 per unit); issue-bound (66% in ncu; XU 44%)")
 
     cfg1 = None
     if not args.no_config1 and rank == 0 and world == 1:
@@ -949,15 +943,15 @@ def main():
         npx1 = float(cfg1["pixels"])
         t32, t64 = cfg1["f32c"]["ms"] * 1e-3, cfg1["f64"]["ms"] * 1e-3
         r32 = roofline_of("fp32", CFG1_F32C_FP32_FLOP_PER_PIXEL, npx1, t32, peak_fp32, "pixel",
-                          "ncu executed FP32 FLOP of grain_dwba_f32c_kernel (plus 554 FP64 per pixel); "
+                          "ncu executed FP32 FLOP of grain_dwba_real_kernel (plus 307 FP64 per pixel); "
                           "the time is the whole simulation (set-up, Fresnel coefficients, grain kernel, sums)")
         xu = CFG1_F32C_XU_PER_PIXEL * npx1 / t32 / 1e9
         r32["sfu"] = {"ops_per_unit": CFG1_F32C_XU_PER_PIXEL, "achieved_gops": xu, "peak_gops": peak_sfu,
                       "frac": xu / peak_sfu, "note": "XU-pipe thread operations (transcendentals and "
-                      "conversions); 29% busy in ncu, the kernel issue-bound (81%)"}
+                      "conversions); 24% busy in ncu, the kernel issue- and latency-bound (54%)"}
         cfg1["f32c"]["roofline"] = r32
         cfg1["f64"]["roofline"] = roofline_of("fp64", CFG1_F64_FLOP_PER_PIXEL, npx1, t64, peak_fp64, "pixel",
-                                              "ncu executed FP64 FLOP of grain_dwba_kernel; the time is "
+                                              "ncu executed FP64 FLOP of grain_dwba_real_kernel; the time is "
                                               "the whole simulation")
 
     cpu = None
@@ -981,18 +975,18 @@ def main():
                        "triangles": ntri, "grid": [NCOL, NROW], "blocks": 4,
                        "evals_per_step": evals, "parallelism": f"replicas x{world}",
                        "l2": "inputs larger than L2 (q-grid 332 MB)",
-                       "launch_shape": {"pixels_per_thread": tuned_p,
-                                        "kernel": "packed FP32x2" if tuned_p < 0 else "scalar",
-                                        "autotuner_ms_8192_triangles":
-                                            {str(k): v for k, v in tune_times.items()}}},
-            "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak_fp32,
-                         "unit": "TFLOP/s", "frac": achieved / peak_fp32,
+                       "launch_shape": {"pixels_per_thread": args.ppt,
+                                        "kernel": "tensor cores (automatic)" if args.ppt == 0 else
+                                                  "packed FP32x2" if args.ppt < 0 else "scalar"}},
+            "roofline": {"bound": "sfu", "achieved": sfu_rate, "peak": peak_sfu,
+                         "unit": "Gop/s", "frac": sfu_rate / peak_sfu,
                          "traffic": TRAFFIC_BYTES_PER_LAUNCH,
                          "traffic_source": TRAFFIC_SOURCE,
-                         "peak_source": "hgx_measure_peaks FFMA probe, sustained 2 s, same GPU",
-                         "flop_per_pixel_triangle": FLOP_PER_PIXEL_TRI,
-                         "sfu": {"achieved_gops": sfu_rate, "peak_gops": peak_sfu,
-                                 "frac": sfu_rate / peak_sfu},
+                         "peak_source": "hgx_measure_peaks __sinf probe, same GPU",
+                         "sfu_per_pixel_triangle": SFU_PER_PIXEL_TRI,
+                         "int8_tensor_tops": INT8_OPS_PER_PIXEL_TRI * n * ntri / (ms_step * 1e-3) / 1e12,
+                         "fp32_form": {"flop_per_pixel_triangle": FLOP_PER_PIXEL_TRI, "achieved_tflops": achieved,
+                                       "of_ffma_probe": achieved / peak_fp32},
                          "hbm_view": hbm_view(ms_step)},
             "peaks": {"fp32_tflops": peak_fp32, "fp64_tflops": peak_fp64, "sfu_gops": peak_sfu,
                       "source": "the library's probes on this GPU (FFMA sustained 2 s, DFMA burst, __sinf)"},

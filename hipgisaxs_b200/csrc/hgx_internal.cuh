@@ -178,7 +178,7 @@ int qgrid_reextend(hgx_qgrid g, double alpha_i, double k0, double dn2_re, double
 // place when nqy and nqz match, else a new one (the old one destroyed).
 int shaped_grid(hgx_ctx c, int nqy, const double* qx, const double* qy, int nqz, const double* qz,
                 hgx_qgrid* out);
-// The same grid for the reference-shaped FP32C form factor with qz in host memory, the 4N qz
+// The same grid for the reference-shaped form factor with qz in host memory, the 4N qz
 // values left for later: when the kept grid has these sizes and the host qz array has a
 // detector-row layout, qx and qy are copied on the context's stream and the row table is read
 // from each row's first q-point of the host array (as row_table_kernel takes it), with the mode

@@ -44,3 +44,24 @@ def test_far_from_the_origin(ctx, po):
     G = po.Grid(70, 3, -1.87, 0.01, 2.0, 3.0, 0.2, 10.0)
     g = hg.QGrid.from_arrays(ctx, G.qx, G.qy, G.qz_ext, 70)
     assert po.rel_err(hg.ff_triangles(ctx, g, sd, None, "f64"), po.ff_approx_triangle(sd, G.qx, G.qy, G.qz_ext)) < TOL64
+
+
+@pytest.mark.parametrize("dn2", [(0.0, 0.0), (6e-6, 4e-8)])
+@pytest.mark.parametrize("ncol", [64, 131])
+def test_reference_shaped_call_while_qz_is_copied(po, ncol, dn2):
+    """From the second call with host arrays of the same sizes on, the FP64 row kernel starts from a
+    row table read on the host while the 4N qz values are copied and checked: bit for bit the
+    device grid's result.  A q-point off its row's value, and blocks that pair only in the rows'
+    first q-points, fail the check and are computed from the full qz."""
+    G = po.Grid(ncol, 9, -2.0, 0.0, 2.0, 3.0, 0.2, 10.0, dn2)
+    sd = cloud(np.random.default_rng(ncol), 150)
+    qz_off, qz_pair = G.qz_ext.copy(), G.qz_ext.copy()
+    qz_off[3 * ncol + ncol // 2] += 0.01
+    qz_pair[2 * G.n + 5 * ncol + 1] *= 1.5
+    ctx = hg.Context(0)
+    for qz in (G.qz_ext, G.qz_ext, qz_off, G.qz_ext, qz_pair, G.qz_ext):
+        want = hg.ff_triangles(ctx, hg.QGrid.from_arrays(ctx, G.qx, G.qy, qz), sd, None, "f64")
+        got = hg.ff_triangles_arrays(ctx, sd, G.qx, G.qy, qz, None, "f64")
+        ok = np.isfinite(want)  # a q-point at q = 0 is 0 / 0
+        assert np.array_equal(ok, np.isfinite(got)) and np.array_equal(got[ok], want[ok])
+    ctx.close()

@@ -177,32 +177,35 @@ __device__ __forceinline__ void dirichlet_pair(double ta, double tb, const CylPi
 }
 
 // ---------------------------------------------------------------- row table ----
-// One warp per (candidate, ROI row): lane 8 k + j takes DWBA block k and the height samples
-// j, j + 8, ...; xor shuffles close the height sums inside each group of 8 lanes and then the
-// block sums across the groups (a fixed tree, so every lane holds the same bits).  The row's
-// scalars of the intensity and its H- and a-derivatives: the centre phase has modulus 1 and
-// drops out of |A|^2.
+// Four ROI rows of a candidate per warp: lane 8 r + 4 b + j takes of row r the pair of DWBA blocks b (0
+// and 3, or 2 and 1, whose qz are opposite: their height sums are conjugates) and the height
+// samples j, j + 4, ...; xor shuffles close the height sums and then the block sums (a fixed tree, so
+// every lane of a row holds the same bits).  The row's scalars of the intensity and its
+// H- and a-derivatives: the centre phase has modulus 1 and drops out of |A|^2.  A row per warp, its
+// lanes on 8 or 16 samples, was mostly idle lanes: this and the tables, 48 regions of 96 to 640 rows, 21 us;
+// with a row per warp 27, with all four blocks' sums and 8 lanes per table node as well 31.
+constexpr int CYL_ROW_LANES = 4;                           // lanes on the samples of a pair
+constexpr int CYL_ROWS_PER_WARP = 16 / CYL_ROW_LANES;
+
 __device__ __forceinline__ void cyl_rows_body(const CylCand& c, int bx, const double2* __restrict__ rowqz,
                                               const double2* __restrict__ rowfc, RowTab* __restrict__ tab) {
-  const int lr = (int)((bx * blockDim.x + threadIdx.x) >> 5);
-  if (lr >= c.nrows) return;  // whole warps
-  const int lane = threadIdx.x & 31, k = lane >> 3;
+  constexpr int L = CYL_ROW_LANES;
+  const int row = (int)((bx * blockDim.x + threadIdx.x) / (2 * L)), lr = min(row, c.nrows - 1);
+  const int lane = threadIdx.x & (2 * L - 1), k = lane / L * 2;
   const int grow = c.row0 + lr;
   const double qz = rowqz[4L * grow + k].x;
   zd G(0, 0), GH(0, 0);
-  for (int j = lane & 7; j < c.nh; j += 8) {
+  for (int j = lane % L; j < c.nh; j += L) {
     double h = c.h[j];
     double x = 0.5 * qz * h;  // sinc(qz h / 2) e^{i qz h / 2} h
     double sx, cx;
     sincos(x, &sx, &cx);
     double sincv = fabs(x) > 1.0e-14 ? sx / x : 1.0 - x * x / 6.0 + x * x * x * x / 120.0;
     G += zd(cx, sx) * (sincv * h);
-    double s2, c2;
-    sincos(2.0 * x, &s2, &c2);
-    GH += zd(c2, s2) * (h / c.H);
+    GH += zd(1.0 - 2.0 * sx * sx, 2.0 * sx * cx) * (h / c.H);  // e^{2ix}
   }
 #pragma unroll
-  for (int o = 1; o < 8; o <<= 1) {
+  for (int o = 1; o < L; o <<= 1) {
     G.x += __shfl_xor_sync(0xffffffffu, G.x, o);
     G.y += __shfl_xor_sync(0xffffffffu, G.y, o);
     GH.x += __shfl_xor_sync(0xffffffffu, GH.x, o);
@@ -211,18 +214,18 @@ __device__ __forceinline__ void cyl_rows_body(const CylCand& c, int bx, const do
   double Sc, dSc;
   const double thc = c.a * c.uc * qz;
   dirichlet(thc, c.rep[2], &Sc, &dSc);
-  const zd f = zd(rowfc[4L * grow + k]) * expi(c.center[2] * qz);
-  zd Q = f * (G * Sc), QH = f * (GH * Sc), Qa = f * (G * (dSc * thc / c.a));
-#pragma unroll
-  for (int o = 8; o < 32; o <<= 1) {
-    Q.x += __shfl_xor_sync(0xffffffffu, Q.x, o);
-    Q.y += __shfl_xor_sync(0xffffffffu, Q.y, o);
-    QH.x += __shfl_xor_sync(0xffffffffu, QH.x, o);
-    QH.y += __shfl_xor_sync(0xffffffffu, QH.y, o);
-    Qa.x += __shfl_xor_sync(0xffffffffu, Qa.x, o);
-    Qa.y += __shfl_xor_sync(0xffffffffu, Qa.y, o);
-  }
-  if (lane == 0) {
+  const zd e = expi(c.center[2] * qz);
+  const double ga = dSc * thc / c.a;  // even in qz, as Sc
+  const zd f = zd(rowfc[4L * grow + k]) * e, fm = zd(rowfc[4L * grow + 3 - k]) * conj(e);
+  const zd T = f * G + fm * conj(G), TH = f * GH + fm * conj(GH);
+  zd Q = T * Sc, QH = TH * Sc, Qa = T * ga;
+  Q.x += __shfl_xor_sync(0xffffffffu, Q.x, L);
+  Q.y += __shfl_xor_sync(0xffffffffu, Q.y, L);
+  QH.x += __shfl_xor_sync(0xffffffffu, QH.x, L);
+  QH.y += __shfl_xor_sync(0xffffffffu, QH.y, L);
+  Qa.x += __shfl_xor_sync(0xffffffffu, Qa.x, L);
+  Qa.y += __shfl_xor_sync(0xffffffffu, Qa.y, L);
+  if (lane == 0 && row < c.nrows) {
     const double K2 = c.K[0] * c.K[0] + c.K[1] * c.K[1];
     RowTab t;
     t.q2 = K2 * norm2(Q);
@@ -236,8 +239,9 @@ __device__ __forceinline__ void cyl_rows_body(const CylCand& c, int bx, const do
 }
 
 // --------------------------------------------------------- radial-sum tables ----
-// A block sums 32 nodes, 8 lanes per node: lane l takes the radius samples l, l + 8, ..., xor
-// shuffles close the sum ((fr, frR) at q = |j - 1| h, as the pixel pass would sum them), except
+// A block sums 32 nodes: a warp takes one radius sample at all of them (so that its lanes' arguments
+// are close and its Bessel functions take one branch), and two warps add the samples in order
+// ((fr, frR) at q = |j - 1| h, as the pixel pass would sum them), except
 // that the q_par -> 0 guard takes the smooth limit (J1(x)/x -> 1/2, J0 -> 1) so that the
 // interpolation near q = 0 is right; pixels that meet the guard sum directly.  Then 29 threads
 // make the cubics of the intervals from node j0 + 1 on: the polynomial in t of the 4-point
@@ -245,33 +249,26 @@ __device__ __forceinline__ void cyl_rows_body(const CylCand& c, int bx, const do
 // a pair (hi, lo), so that no rounding of a node, common to every pixel near that q_par, reaches
 // the intensity (the other terms vanish at the nodes and are a few per cent of it between them).
 constexpr int CYL_PREP_THREADS = 256;
-constexpr int CYL_CELLS = CYL_PREP_THREADS / 8 - 3;
+constexpr int CYL_CELLS = 32 - 3;
 
 __device__ __forceinline__ void cyl_table_body(const CylCand& c, int bx, double h, CylCell* __restrict__ table) {
-  __shared__ double s_node[CYL_PREP_THREADS / 8][2];
-  const int n = threadIdx.x >> 3, l = threadIdx.x & 7, j = bx * CYL_CELLS + n;
-  const double qp = fabs((double)(j - 1) * h);
-  double fr = 0.0, frR = 0.0;
-  for (int i = l; i < c.nr; i += 8) {
+  __shared__ double s_term[CYL_MAXS][2][32];
+  __shared__ double s_node[32][2];
+  const int n = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const double qp = fabs((double)(bx * CYL_CELLS + n - 1) * h);
+  for (int i = w; i < c.nr; i += CYL_PREP_THREADS / 32) {
     const double r = c.r[i];
     const double x = qp * r;
-    const double two_pi_r = 2.0 * PI_D * r;
-    if (x * x > 1.0e-13) {
-      fr += two_pi_r * r * j1(x) / x;
-      frR += two_pi_r * r * j0(x);
-    } else {
-      fr += two_pi_r * r * 0.5;
-      frR += two_pi_r * r;
-    }
+    const double two_pi_r2 = 2.0 * PI_D * r * r;
+    const bool far = x * x > 1.0e-13;
+    s_term[i][0][n] = far ? two_pi_r2 * j1(x) / x : two_pi_r2 * 0.5;
+    s_term[i][1][n] = far ? two_pi_r2 * j0(x) : two_pi_r2;
   }
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) {
-    fr += __shfl_xor_sync(0xffffffffu, fr, o);
-    frR += __shfl_xor_sync(0xffffffffu, frR, o);
-  }
-  if (l == 0) {
-    s_node[n][0] = fr;
-    s_node[n][1] = frR / c.R;
+  __syncthreads();
+  if (w < 2) {
+    double v = 0.0;
+    for (int i = 0; i < c.nr; ++i) v += s_term[i][w][n];
+    s_node[n][w] = w ? v / c.R : v;
   }
   __syncthreads();
   const int cell = bx * CYL_CELLS + 1 + (int)threadIdx.x;
@@ -291,8 +288,8 @@ __device__ __forceinline__ void cyl_table_body(const CylCand& c, int bx, double 
   }
 }
 
-// The per-evaluation set-up in one launch: blocks [0, row_blocks) build the row table (a warp
-// per ROI row), the rest (FP32C only) the radial-sum tables; grid y = candidate.
+// The per-evaluation set-up in one launch: blocks [0, row_blocks) build the row table (four
+// ROI rows per warp), the rest (FP32C only) the radial-sum tables; grid y = candidate.
 __global__ void cyl_prep_kernel(const CylCand* __restrict__ cands, int row_blocks,
                                 const double2* __restrict__ rowqz, const double2* __restrict__ rowfc,
                                 RowTab* __restrict__ tab, double h, CylCell* __restrict__ table) {
@@ -801,9 +798,9 @@ static int cyl_enqueue(hgx_cyl_batch_s* b, bool with_counts, bool with_intensity
                            cudaMemcpyHostToDevice, st));
   int maxrows = 0;
   for (int i = 0; i < b->ncand; ++i) maxrows = std::max(maxrows, b->rois[4 * i + 2]);
-  // row table (a warp per row) and, in FP32C, the radial-sum tables
+  // row table (four rows per warp) and, in FP32C, the radial-sum tables
   // (CYL_CELLS intervals per block, the last one CYL_NTAB - 3) in one launch
-  const int row_blocks = (maxrows + CYL_PREP_THREADS / 32 - 1) / (CYL_PREP_THREADS / 32);
+  const int rpb = CYL_PREP_THREADS / 32 * CYL_ROWS_PER_WARP, row_blocks = (maxrows + rpb - 1) / rpb;
   const int table_blocks = b->precision == HGX_F32C ? (CYL_NTAB - 3 + CYL_CELLS - 1) / CYL_CELLS : 0;
   cyl_prep_kernel<<<dim3(row_blocks + table_blocks, b->ncand), CYL_PREP_THREADS, 0, st>>>(
       (const CylCand*)b->d_cands.p, row_blocks, b->grid->rowqz, (const double2*)b->d_rowfc.p,

@@ -1141,15 +1141,25 @@ static int prepare_tiles(hgx_ctx c, const double* sd, int ntri, const Rot9& R, b
   return HGX_OK;
 }
 
-// The tensor-core row kernel takes row grids of any width: its unit is 128 columns, but even a
-// narrow grid is faster there (16 x 16 x 1,280 triangles: 0.059 against 0.122 ms; 48 x 256: 0.090
-// against 0.123; 130 x 512 x 4,800: 0.52 against 0.90; complex blocks 1.4 to 4.4 times faster at
-// every size tried).  The FP32 row kernel keeps one corner: real blocks, at most 64 columns and
-// rows that fill its two CTAs per SM at one pixel per thread (64 x 1024 x 4,800: 0.515 against
-// 0.560 ms; at 300 rows 0.320 against 0.245, from 8 CTAs of 4 rows per 4 SMs on 3.4 against 1.07).
-static bool rows_mma_pays(hgx_ctx c, hgx_qgrid g) {
-  const int ctas = (g->nrow + 3) / 4;
-  return !(g->mode == 1 && g->ncol <= 64 && 4 * ctas >= 7 * c->sm_count && ctas < 2 * c->sm_count);
+// Which row kernel an untuned FP32C call takes.  Complex blocks: always the tensor cores (1.4 to 4.4 times
+// faster at every size tried).  Real blocks: the estimated times in us, from 712 sizes of 16 to 1024
+// columns, 60 to 2048 rows and 100 to 4,800 triangles.  A CTA of the FP32 kernel takes 21.5 per tile (however full)
+// and pixel per thread, CTAs that share an SM one after another as far as throughput goes; a CTA of
+// the tensor-core kernel (128 columns of a row, one per SM) 7.2 to start and to end, 1.5 more for each
+// further tile and 0.0108 per triangle.  So the FP32 kernel keeps single full tiles on large grids and, up
+// to a few thousand triangles, grids of at most 64 columns (whose other half the tensor-core kernel pads)
+// with rows for about two CTAs per SM: 64 x 800 x 506 0.062 against 0.095 ms, 64 x 1024 x 1,000 0.133
+// / 0.178, 150 x 400 x 506 0.076 / 0.088.  On the other side 64 x 60 x 506 0.037 / 0.042, 128 x 300
+// x 506 0.074 / 0.082, 48 x 256 x 1,280 0.090 / 0.123, 130 x 512 x 4,800 0.52 / 0.90.  The margin leaves ties to
+// the tensor cores; over the 712 sizes the choice is at most 6% off the faster kernel where it
+// takes the tensor cores and 10% where it takes the FP32 kernel.
+static bool rows_mma_pays(hgx_ctx c, hgx_qgrid g, int ntri) {
+  if (g->mode != 1) return true;
+  const RowShape sh = row_shape(g->nrow, g->ncol, c->sm_count, 4);
+  const double tiles = (ntri + TILE - 1) / TILE, sms = c->sm_count;
+  const double fp32 = ceil((double)sh.grid.x * sh.grid.y / sms) * tiles * 21.5 * (sh.P == 4 ? 3.8 : sh.P);
+  const double mma = ceil((double)g->nrow * ((g->ncol + 127) / 128) / sms) * (7.2 + 1.5 * (tiles - 1) + 0.0108 * ntri);
+  return !(fp32 < 0.9 * mma);
 }
 
 int ff_triangles_device(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, const double* rot9,
@@ -1169,7 +1179,7 @@ int ff_triangles_device(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, cons
     HGX_CUDA(cudaGetLastError());
     return HGX_OK;
   }
-  if (want_p == 0 && g->tuned_p == 0 && g->mode != 0 && rows_mma_pays(c, g)) {
+  if (want_p == 0 && g->tuned_p == 0 && g->mode != 0 && rows_mma_pays(c, g, ntri)) {
     if (row_shape(g->nrow, g->ncol, c->sm_count, 4).grid.y > 65535u)
       return fail(HGX_ERR_INVALID_ARG, "hgx_ff_triangles: too many detector rows for one launch");
     TilePrep t;

@@ -82,3 +82,12 @@ def test_a_triangle_that_is_not_finite_is_not_hidden(ctx, po, col, value):
     qx, qy, qz = detector(po, 33, 3, "real")
     g = hg.QGrid.from_arrays(ctx, qx, qy, qz, 33)
     assert not np.isfinite(hg.ff_triangles(ctx, g, sd, None, "f32c")).any()
+
+
+@pytest.mark.parametrize("ncol,nrow,ntri", [(64, 800, 300), (64, 60, 506), (150, 400, 506), (150, 400, 513), (30, 1030, 600)])
+def test_both_sides_of_the_kernel_choice(ctx, po, ncol, nrow, ntri):
+    """Real blocks near the sizes at which the automatic choice goes from one row kernel to the other."""
+    sd = cloud(np.random.default_rng(ncol + ntri), ntri)
+    qx, qy, qz = detector(po, ncol, nrow, "real")
+    g = hg.QGrid.from_arrays(ctx, qx, qy, qz, ncol)
+    assert po.rel_err(hg.ff_triangles(ctx, g, sd, None, "f32c"), po.ff_approx_triangle(sd, qx, qy, qz)) < TOL32

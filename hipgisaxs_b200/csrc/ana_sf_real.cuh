@@ -6,11 +6,12 @@
 //
 // Lattice structure factor: for a real angle the reference's principal-branch complex powers
 //   pow(e, (1 - N)/2) (1 - pow(e, N)) / (1 - e),  e = e^{i theta}  (src/sf/sf.cpp:164-246)
-// are sin(N theta_r / 2) / sin(theta_r / 2) with theta_r the principal angle of e; on the b axis
-// the numerator takes the unreduced theta, which for a non-integer N adds the phase
-// e^{i pi k (N - 1)}, theta = theta_r + 2 pi k.  N is returned at theta_r = 0, where the reference's
-// guard takes N.  Two sines instead of five complex exponentials, four powers and three divisions;
-// angles in turns, so that their reduction is exact.
+// are sin(N theta_r / 2) / sin(theta_r / 2) with theta_r the principal angle of e.  On the b axis
+// the reference's numerator is 1 - e^{i N theta} of the unreduced theta = theta_r + 2 pi k: the same
+// for a whole N, sin(N theta / 2) / sin(theta_r / 2) e^{i pi k N} for another (dirichlet_b_real,
+// b_phase_real).  N is returned at theta_r = 0, where the reference's guard takes N.  Two sines
+// instead of five complex exponentials, four powers and three divisions; angles in turns, so that
+// their reduction is exact.
 //
 // Form factors: sinc(x) e^{ix} terms as one sincos; the cylinder's evenly stepped heights in
 // closed form (ana_sf_f32.cuh) where the samples step to rounding (FP64: prog == 2).
@@ -75,27 +76,40 @@ __device__ __forceinline__ float sinc_real(double x, float sinx) { return sinc_f
 
 // A lattice factor as num / den at the angle of `u` turns; N itself within 1e-13 turn of a whole
 // one, where the ratio is N to rounding (the products of two denominators then stay in range).
+// FULL: the numerator takes the unreduced angle, and N is the value at a whole number of turns only
+// (elsewhere near one the ratio is far from N unless that number is 0).
 template <typename T>
 struct Ratio {
   T num, den;
 };
 template <typename T>
-__device__ __forceinline__ Ratio<T> dirichlet_real(double u, double N);
+__device__ __forceinline__ Ratio<T> dirichlet_real(double u, double N, bool full = false);
 template <>
-__device__ __forceinline__ Ratio<double> dirichlet_real<double>(double u, double N) {
+__device__ __forceinline__ Ratio<double> dirichlet_real<double>(double u, double N, bool full) {
   const double t = u - round_fp64(u), h = 0.5 * t;
-  const double n = sin_turns(N * h), d = sin_quarter_turn(h);
-  const bool zero = fabs(t) < 1e-13;
+  const double n = sin_turns(N * (full ? 0.5 * u : h)), d = sin_quarter_turn(h);
+  const bool zero = full ? t == 0.0 : fabs(t) < 1e-13;
   return Ratio<double>{zero ? N : n, zero ? 1.0 : d};
 }
 template <>
-__device__ __forceinline__ Ratio<float> dirichlet_real<float>(double u, double N) {
+__device__ __forceinline__ Ratio<float> dirichlet_real<float>(double u, double N, bool full) {
   const double t = u - round_fp64(u);
-  const double v = N * t, kv = v + RND52;  // nearest integer in the low mantissa bits
+  const double v = N * (full ? u : t), kv = v + RND52;  // nearest integer in the low mantissa bits
   const float n = sin_half_turn((float)(v - (kv - RND52))), d = sin_half_turn((float)t);
   const float sn = __int_as_float(__float_as_int(n) ^ (__double2loint(kv) << 31));
-  const bool zero = fabs(t) < 1e-13;
+  const bool zero = full ? t == 0.0 : fabs(t) < 1e-13;
   return Ratio<float>{zero ? (float)N : sn, zero ? 1.0f : d};
+}
+
+// The b axis' factor, and its phase where N is not whole.
+template <typename T>
+__device__ __forceinline__ Ratio<T> dirichlet_b_real(double u, double N) {
+  return dirichlet_real<T>(u, N, N != round_fp64(N));
+}
+template <typename T>
+__device__ __forceinline__ cx<T> b_phase_real(double u, double N) {
+  const double k = round_fp64(u);
+  return expi_turns_real<T>(u == k ? 0.0 : 0.5 * k * N);
 }
 
 // The cylinder's radial sum over its samples (unweighted), ff_ana_cylinder.cpp:34-42,100-117.

@@ -397,7 +397,8 @@ __global__ void __launch_bounds__(128, 4) grain_dwba_real_kernel(FusedArgs a) {
         }
       } else if (G.flat) {
         const Ratio<T> ra = dirichlet_real<T>(fma(qx, G.a[0], qy * G.a[1]), G.rep[0]);
-        const Ratio<T> rb = dirichlet_real<T>(fma(qx, G.b[0], fma(qy, G.b[1], G.b0)), G.rep[1]);
+        // (the phase of a b repetition that is not whole is common to the blocks)
+        const Ratio<T> rb = dirichlet_b_real<T>(fma(qx, G.b[0], fma(qy, G.b[1], G.b0)), G.rep[1]);
         ab = quotient(ra.num * rb.num, ra.den * rb.den);
         cx<T> v[4];
 #pragma unroll
@@ -421,10 +422,10 @@ __global__ void __launch_bounds__(128, 4) grain_dwba_real_kernel(FusedArgs a) {
           const cx<T> fk = k == 0 ? f[0] : k == 1 ? f[1] : k == 2 ? f[2] : f[3];
           const double ub = fma(qx, G.b[0], fma(qy, G.b[1], fma(q, G.b[2], G.b0)));
           const Ratio<T> ra = dirichlet_real<T>(fma(qx, G.a[0], fma(qy, G.a[1], q * G.a[2])), G.rep[0]);
-          const Ratio<T> rb = dirichlet_real<T>(ub, G.rep[1]);
+          const Ratio<T> rb = dirichlet_b_real<T>(ub, G.rep[1]);
           const Ratio<T> rc = dirichlet_real<T>(fma(qx, G.c[0], fma(qy, G.c[1], q * G.c[2])), G.rep[2]);
           cx<T> v = (quotient(ra.num, ra.den) * quotient(rb.num, rb.den) * quotient(rc.num, rc.den)) * fk;
-          if (G.rep[1] != round_fp64(G.rep[1])) v = v * expi_turns_real<T>(0.5 * round_fp64(ub) * (G.rep[1] - 1.0));
+          if (G.rep[1] != round_fp64(G.rep[1])) v = v * b_phase_real<T>(ub, G.rep[1]);
           if (G.d[0] != 0.0 || G.d[1] != 0.0 || G.d[2] != 0.0)
             v = v * expi_turns_real<T>(fma(qx, G.d[0], fma(qy, G.d[1], q * G.d[2])));
           sum = sum + v;

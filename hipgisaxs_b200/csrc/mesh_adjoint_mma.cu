@@ -56,6 +56,10 @@ constexpr int BWM_SUMS = BWM_SUB * 6 * 128 * 8;
 constexpr int BWM_NREC = 4;                   // items whose records are held
 constexpr int BWM_SMEM = BWM_NST * BWM_STAGE + BWM_NREC * BWM_REC * 4 + BWM_SUMS;
 constexpr int BWM_D = BWM_ND * BWM_NP;        // accumulator columns, two ranges
+// The combined sums are taken in units of 2^36 and the scales times 2^36 (about half the column's
+// largest modulus), so that neither leaves the range of FP32 where the moduli do not.
+constexpr float BWM_S36 = 1.0f / 68719476736.0f;
+constexpr double BWM_UNIT = V_UNIT / 65536.0 * 68719476736.0;
 
 // The digit planes of four integers b_i = w_i - 0x80808080, |b_i| <= 0x7f7f7f7f.
 __device__ __forceinline__ void signed_digits4(const uint32_t (&w)[4], uint32_t (&dig)[4]) {
@@ -73,6 +77,12 @@ __device__ __forceinline__ float moment(int j, float qx, float qy) {
   return j < 2 ? qx : j < 4 ? qy : j < 6 ? 1.f : j < 8 ? qx * qx : j < 10 ? qx * qy : qy * qy;
 }
 
+// |x + i y|, also where the squares leave FP32's range.
+__device__ __forceinline__ float modulus(float x, float y) {
+  const float m = fmaxf(fabsf(x), fabsf(y));
+  return m > 1e-15f && m < 1e15f ? sqrtf(x * x + y * y) : hypotf(x, y);
+}
+
 // Per item (one CTA): the in-plane q of its pixels as the digit makers read them (pairs, then the
 // largest |q_par|), and the largest modulus of every seed column.
 __global__ void __launch_bounds__(256) bwm_item_kernel(BwmArgs a, int row0) {
@@ -86,7 +96,7 @@ __global__ void __launch_bounds__(256) bwm_item_kernel(BwmArgs a, int row0) {
   const float4 none = make_float4(0, 0, 0, 0), s[2] = {in ? a.seeds[2 * p] : none, in ? a.seeds[2 * p + 1] : none};
 #pragma unroll
   for (int pr = 0; pr < 2; ++pr) {
-    float mp = sqrtf(s[pr].x * s[pr].x + s[pr].y * s[pr].y), mm = sqrtf(s[pr].z * s[pr].z + s[pr].w * s[pr].w);
+    float mp = modulus(s[pr].x, s[pr].y), mm = modulus(s[pr].z, s[pr].w);
     if (!isfinite(mp)) mp = INFINITY;  // the gradient is then not finite either
     if (!isfinite(mm)) mm = INFINITY;
 #pragma unroll
@@ -110,7 +120,7 @@ __global__ void __launch_bounds__(256) bwm_item_kernel(BwmArgs a, int row0) {
   if (i < 25) {
     float m = s_max[0][i];
     for (int k = 1; k < 8; ++k) m = fmaxf(m, s_max[k][i]);
-    if (i < 24) a.colmax[(size_t)item * 24 + i] = fmaxf(m, 1e-30f);  // keeps both scales in range
+    if (i < 24) a.colmax[(size_t)item * 24 + i] = fmaxf(m, 0x1p-124f);  // keeps both scales in range
     else {
       float* e = a.xy + (size_t)item * (w * 2 + 4) + w * 2;
       e[0] = m;
@@ -156,11 +166,13 @@ __global__ void __launch_bounds__(256) bwm_seed_kernel(BwmArgs a, int row0) {
   for (int j = 0; j < 16; ++j) {
     uint32_t x[4], dig[BWM_ND] = {0, 0, 0, 0};
     if (j < 12) {
-      const float sc = (float)(B_SCALE * 256.0 / (double)a.colmax[(size_t)item * 24 + 12 * pr + j]);
+      // two factors where one would leave FP32's range
+      const float top = a.colmax[(size_t)item * 24 + 12 * pr + j], up = top < 0x1p-60f ? 0x1p64f : 1.f;
+      const float sc = (float)(B_SCALE * 256.0 / ((double)top * (double)up));
       int hi = 0, lo = 0;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int b = __float2int_rn(moment(j, q[i][0], q[i][1]) * h[i][(j < 4 ? 0 : 2) + (j & 1)] * sc);
+        const int b = __float2int_rn(moment(j, q[i][0], q[i][1]) * h[i][(j < 4 ? 0 : 2) + (j & 1)] * up * sc);
         hi += b >> 8;
         lo += b & 255;
         x[i] = (uint32_t)b + 0x80808080u;
@@ -191,8 +203,8 @@ __global__ void __launch_bounds__(256) bwm_seed_kernel(BwmArgs a, int row0) {
     const float top = a.colmax[(size_t)item * 24 + c];
     uint32_t* rec = a.rec + cell * BWM_REC + c;
     rec[0] = (uint32_t)(off >> 10);
-    rec[24] = __float_as_uint(top == INFINITY ? NAN : (float)((double)top * (V_UNIT / 65536.0)));
-    rec[48] = __float_as_uint((float)((int)(off & 1023) << 6));
+    rec[24] = __float_as_uint(top == INFINITY ? NAN : (float)((double)top * BWM_UNIT));
+    rec[48] = __float_as_uint((float)((int)(off & 1023) << 6) * BWM_S36);
   }
 }
 
@@ -213,8 +225,10 @@ __device__ __forceinline__ void bwm_add(uint32_t d_tm, const uint32_t* rec, doub
       for (int j = 0; j < 8; ++j) {
         const int c = 12 * pr + 8 * h + j;
         if (8 * h + j < 12) {
-          const float lo = fmaf((float)(int)d[16 + j], 256.f, (float)(int)d[24 + j] - __uint_as_float(rec[48 + c]));
-          f[8 * h + j] = fmaf((float)(int)(d[j] * 256u + d[8 + j] - rec[c]), 65536.f, lo) * __uint_as_float(rec[24 + c]);
+          const float lo = fmaf((float)(int)d[16 + j], 256.f * BWM_S36,
+                                fmaf((float)(int)d[24 + j], BWM_S36, -__uint_as_float(rec[48 + c])));
+          f[8 * h + j] = fmaf((float)(int)(d[j] * 256u + d[8 + j] - rec[c]), 65536.f * BWM_S36, lo) *
+                         __uint_as_float(rec[24 + c]);
         }
       }
     }

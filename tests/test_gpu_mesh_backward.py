@@ -49,3 +49,19 @@ def test_wide_phases(ctx, po):
     V, F = meshes.icosphere(30.0, 3)
     got, ref = gradients(ctx, po, 140, 3, V, F)
     assert po.rel_err(got, ref) < 1e-4
+
+
+@pytest.mark.parametrize("unit", [1e-18, 1e-15, 1e20])
+def test_units_of_the_counts(ctx, po, unit):
+    """Counts and scale in other units: seeds of 1e-31, 1e-25 and 1e21, whose squares leave FP32's range."""
+    V, F = meshes.icosphere(8.0, 2, jitter=0.2, seed=3)
+    G = po.Grid(140, 3, -2.0, 0.0, 2.0, 3.0, 0.2, 10.0)
+    g = hg.QGrid.create(ctx, 140, 3, -2.0, 0.0, 2.0, 3.0, G.alpha_i, G.k0)
+    rowfc = model.propagation_coeffs(ctx, g, [SUB], G.k0, G.alpha_i, 0, per_row=True)
+    inten = fitting.mesh_chi2_grad(ctx, g, V, F, rowfc, DN2, None, None, 1.0, 1.0, None, want_grad=False,
+                                   want_intensity=True, precision="f64")[2]
+    scale = unit * 1e4 / inten.max()
+    counts = scale * inten * np.random.default_rng(2).uniform(0.2, 0.6, G.n)
+    got, ref = [fitting.mesh_chi2_grad(ctx, g, V, F, rowfc, DN2, counts, None, scale, 1.0, None, precision=p)[1]
+                for p in ("f32c", "f64")]
+    assert np.isfinite(ref).all() and np.abs(ref).max() > 0 and po.rel_err(got, ref) < 1e-4

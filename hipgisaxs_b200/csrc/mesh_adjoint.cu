@@ -581,15 +581,15 @@ int hgx_mesh_chi2_grad_ex(hgx_ctx c, hgx_qgrid g, int nv, const double* verts, i
     chunks = (g->nrow + rpc - 1) / rpc;
     int done = HGX_ERR_NO_MEMORY;
     if (plan.slabs) {
-      // every slab has the same number of row ranges; the last one may have fewer rows than ranges
-      const int parts = plan.slabs * plan.splits;
-      HGX_TRY(w.bwpart.reserve(sizeof(double) * 6 * (size_t)nf * std::max(parts, chunks)));
-      HGX_CUDA(cudaMemsetAsync(w.bwpart.p, 0, sizeof(double) * 6 * (size_t)nf * parts, st));
-      BwmArgs ba{tv.tiles, tv.anchors, tv.perm, nf, tv.ntiles, (const float4*)seeds.p, g->qx, g->qy, g->rowqz,
-                 g->nrow, g->ncol, (double*)w.bwpart.p};
-      done = bwm_run(c, plan, ba);
-      if (done == HGX_OK) chunks = parts;
-      else if (done != HGX_ERR_NO_MEMORY) return done;  // without room for the seed digits: the FP32 kernel
+      // without room for the partial sums or the seed digits: the FP32 kernel
+      done = w.bwpart.reserve(sizeof(double) * 6 * (size_t)nf * plan.splits);
+      if (done == HGX_OK) {
+        BwmArgs ba{tv.tiles, tv.anchors, tv.perm, nf, tv.ntiles, (const float4*)seeds.p, g->qx, g->qy, g->rowqz,
+                   g->nrow, g->ncol, (double*)w.bwpart.p};
+        done = bwm_run(c, plan, ba);
+      }
+      if (done == HGX_OK) chunks = plan.splits;
+      else if (done != HGX_ERR_NO_MEMORY) return done;
     }
     HGX_TRY(gtri.reserve(sizeof(double) * 6 * nf));
     DevBuf& bwpart = w.bwpart;

@@ -15,7 +15,7 @@ struct BwmArgs {
   const double* qy;
   const double2* rowqz;      // nrow x 4
   int nrow, ncol;
-  double* partial;           // [slabs x splits][ntri][6]
+  double* partial;           // [splits][ntri][6], the slabs' sums added in order
   // set by bwm_run: items per row, 32-pixel chunks per item, and the slab's arrays
   int nch, nck;
   unsigned char* b;

@@ -256,7 +256,7 @@ __device__ __forceinline__ void bwm_add(uint32_t d_tm, const uint32_t* rec, doub
 
 // Every wait is bounded, as in ff_tri_mma_kernel: a thread whose wait gives up goes on without
 // waiting (all addresses stay in range) and the error word says so.
-__global__ void __launch_bounds__(BWM_THREADS, 1) bwm_kernel(BwmArgs a, int row0, int nrows, int part0) {
+__global__ void __launch_bounds__(BWM_THREADS, 1) bwm_kernel(BwmArgs a, int row0, int nrows) {
   constexpr int SUB = BWM_SUB, NST = BWM_NST;
   extern __shared__ __align__(1024) unsigned char s_mem[];
   __shared__ __align__(8) uint64_t s_full[NST], s_ready[SUB], s_used[SUB], s_free[2], s_done;
@@ -414,12 +414,12 @@ __global__ void __launch_bounds__(BWM_THREADS, 1) bwm_kernel(BwmArgs a, int row0
     const int t = a.perm[(size_t)tile * TILE + quarter * 128 + lt];
     if (t >= 0) {
       const double* sums = s_sums + lt;
-      double* dst = a.partial + ((size_t)(part0 + blockIdx.y) * a.ntri + t) * 6;
+      double* dst = a.partial + ((size_t)blockIdx.y * a.ntri + t) * 6;
 #pragma unroll
       for (int k = 0; k < 6; ++k) {
         double v = 0.0;
         for (int w = 0; w < SUB; ++w) v += sums[(w * 6 + k) * 128];
-        dst[k] = v;
+        dst[k] = row0 ? dst[k] + v : v;  // a later slab adds to the earlier ones' sums
       }
     }
   }
@@ -428,6 +428,7 @@ __global__ void __launch_bounds__(BWM_THREADS, 1) bwm_kernel(BwmArgs a, int row0
 
 // -------------------------------------------------------------------- host ----
 constexpr size_t BWM_SLAB_BYTES = (size_t)1 << 30;  // seed digits held at a time
+constexpr size_t BWM_PART_BYTES = (size_t)64 << 20;  // partial sums (one row range's at least)
 
 // Grids of up to 128 columns stay with the FP32 kernel: an item needs a chunk per warpgroup.  From 129
 // on this pass is the faster one at every size tried (whole call, both with the same forward: 130 x 2 x
@@ -443,10 +444,12 @@ BwmPlan bwm_plan(hgx_ctx c, hgx_qgrid g, int ntiles, int ntri) {
   p.rows = (int)std::max<size_t>(1, std::min<size_t>(g->nrow, BWM_SLAB_BYTES / row));
   p.slabs = (g->nrow + p.rows - 1) / p.rows;
   p.rows = (g->nrow + p.slabs - 1) / p.slabs;  // slabs of equal size
-  // row ranges per group of triangles: whole waves of CTAs, a CTA's own cost about one item
+  // row ranges per group of triangles: whole waves of CTAs, a CTA's own cost about one item.  The slabs
+  // share the ranges' partial sums, so that these do not grow with the number of slabs (itself
+  // proportional to pixels x triangles).
   const int groups = (ntri + 127) / 128;
   double best = 0.0;
-  for (int k = 1; k <= p.rows && k <= 64; ++k) {
+  for (int k = 1; k <= p.rows && k <= 64 && (k == 1 || k * sizeof(double) * 6 * (size_t)ntri <= BWM_PART_BYTES); ++k) {
     const double cost = (double)((groups * (long)k + c->sm_count - 1) / c->sm_count) *
                         ((double)((p.rows + k - 1) / k) * p.nch + 1.5);
     if (k == 1 || cost < best) {
@@ -482,7 +485,8 @@ int bwm_run(hgx_ctx c, const BwmPlan& p, BwmArgs a) {
     if (n <= 0) break;
     bwm_item_kernel<<<dim3(p.nch, n), 256, 0, st>>>(a, row0);
     bwm_seed_kernel<<<dim3(a.ntiles, n * p.nch), 256, p.nck * BWM_IMG_CHUNK, st>>>(a, row0);
-    bwm_kernel<<<dim3(groups, std::min(p.splits, n)), BWM_THREADS, BWM_SMEM, st>>>(a, row0, n, s * p.splits);
+    // (the last slab may have fewer rows than ranges, the first one has at least as many)
+    bwm_kernel<<<dim3(groups, std::min(p.splits, n)), BWM_THREADS, BWM_SMEM, st>>>(a, row0, n);
     HGX_CUDA(cudaGetLastError());
   }
   return HGX_OK;

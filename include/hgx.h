@@ -394,7 +394,9 @@ int hgx_mesh_to_shape_def(hgx_ctx ctx, int nv, const double* verts, int nf, cons
  * FP32C mesh form factor of the rotated mesh (rot9 or NULL); rowfc: per-row Fresnel
  * coefficients (nrow x 4); chi^2 = sum mask (scale I - counts)^2 / max(counts, 1).
  * Outputs: chi2 (host double), grad_verts (nv x 3, may be NULL), intensity (N, may be
- * NULL).  The grid must be a DWBA grid with real qz constant along rows. */
+ * NULL).  The grid must be a DWBA grid with real qz constant along rows.  On grids wider than
+ * 128 columns the context keeps up to 1 GiB of seed digits (the same block as the form factor's row
+ * factors) and, on any, partial sums of 48 bytes per face and row range (64 MiB or one range). */
 int hgx_mesh_chi2_grad(hgx_ctx ctx, hgx_qgrid g, int nv, const double* verts, int nf,
                        const int* faces, const double* rot9, const double* rowfc,
                        double dn2_re, double dn2_im, double weight, const double* counts,

@@ -65,3 +65,26 @@ def test_units_of_the_counts(ctx, po, unit):
     got, ref = [fitting.mesh_chi2_grad(ctx, g, V, F, rowfc, DN2, counts, None, scale, 1.0, None, precision=p)[1]
                 for p in ("f32c", "f64")]
     assert np.isfinite(ref).all() and np.abs(ref).max() > 0 and po.rel_err(got, ref) < 1e-4
+
+
+@pytest.mark.parametrize("ncol,nrow,f64", [(160, 200, True), (2048, 96, False)])  # 5 and 32 slabs
+def test_slabs_of_seed_digits_share_their_partial_sums(po, ncol, nrow, f64):
+    """Several slabs of rows: their sums add up, and the call's device memory stays below the 1 GiB of
+    seed digits, 64 MiB of partial sums and some 150 MiB of arrays that go with the pixels or the faces."""
+    import torch
+    V, F = meshes.star_mesh(15.0, 500, 328)  # 327,000 faces
+    ctx = hg.Context(0)
+    gradients(ctx, po, 160, 2, V[:3], np.array([[0, 1, 2]], dtype=np.int32))  # loads the kernels
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    G = po.Grid(ncol, nrow, -2.0, 0.0, 2.0, 3.0, 0.2, 10.0)
+    g = hg.QGrid.create(ctx, ncol, nrow, -2.0, 0.0, 2.0, 3.0, G.alpha_i, G.k0)
+    rowfc = model.propagation_coeffs(ctx, g, [SUB], G.k0, G.alpha_i, 0, per_row=True)
+    counts = np.random.default_rng(4).uniform(1.0, 2.0, G.n)
+    args = (ctx, g, V, F, rowfc, DN2, counts, None, 1.0, 1.0, None)
+    got = fitting.mesh_chi2_grad(*args, precision="f32c")[1]
+    used = free - torch.cuda.mem_get_info()[0]
+    ref = fitting.mesh_chi2_grad(*args, precision="f64")[1] if f64 else got
+    ctx.close()
+    assert used < (1 << 30) + (64 << 20) + (150 << 20)
+    assert po.rel_err(got, ref) < 1e-4

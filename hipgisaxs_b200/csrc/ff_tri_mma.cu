@@ -518,10 +518,8 @@ __global__ void __launch_bounds__(MmaShape<U>::THREADS, 1) ff_tri_mma_kernel(Mma
         unread = -1;
       }
     }
-    if (unread >= 0) {
-      wait_used();
-      read_back(unread);
-    }
+    wait_used();  // no arrival is left under way when the block ends
+    if (unread >= 0) read_back(unread);
   } else {
     // one warp for the products with cos, one for those with sin (independent accumulators); the
     // whole warp walks the chunks so that the operands stay in uniform registers

@@ -350,10 +350,8 @@ __global__ void __launch_bounds__(BWM_THREADS, 1) bwm_kernel(BwmArgs a, int row0
       }
       if (ch == nck - 1) unread = i;
     }
-    if (unread >= 0) {
-      wait_used();
-      read_back(unread);
-    }
+    wait_used();  // no arrival is left under way when the block ends
+    if (unread >= 0) read_back(unread);
   } else {
     int k = 0, use = 0;
     if (elect_one())
@@ -378,7 +376,7 @@ __global__ void __launch_bounds__(BWM_THREADS, 1) bwm_kernel(BwmArgs a, int row0
             mma_s8_ts(dc + 2 * BWM_NP, av + 24 * t + 16, b, idesc_s8(2 * BWM_NP), 1);
           }
           mma_commit(&s_used[k]);
-          if (ch == nck - 1) mma_commit(&s_done);
+          if (ch == nck - 1 && i + 1 < ni) mma_commit(&s_done);  // waited for below, in the next item
         }
         __syncwarp();
         // Two chunks on, the last item's products are done and its pixels were read before: its
@@ -408,6 +406,7 @@ __global__ void __launch_bounds__(BWM_THREADS, 1) bwm_kernel(BwmArgs a, int row0
       atomicOr(a.err, (unsigned)DEV_ERR_WAIT_TIMEOUT);
       for (int i = ni > NST ? ni - NST : 0; i < ni; ++i) mbar_wait(&s_full[i % NST], (i / NST) & 1);
       for (int k = 0; k < SUB; ++k) mbar_wait(&s_used[k], ((ni * nck - 1 - k) / SUB) & 1);
+      if (ni > 1) mbar_wait(&s_done, (ni - 2) & 1);
     }
     __syncthreads();
   } else if (wg == 0) {

@@ -88,3 +88,12 @@ def test_slabs_of_seed_digits_share_their_partial_sums(po, ncol, nrow, f64):
     ctx.close()
     assert used < (1 << 30) + (64 << 20) + (150 << 20)
     assert po.rel_err(got, ref) < 1e-4
+
+
+@pytest.mark.parametrize("ncol,nrow,nfaces", [(129, 2, 128), (160, 148, 129), (300, 70, 1280)])
+def test_blocks_that_follow_one_another_leave_each_other_alone(ctx, po, ncol, nrow, nfaces):
+    """One item per block, and several with fewer and more blocks than SMs: the same bits on every call."""
+    V, F = meshes.icosphere(8.0, 3, jitter=0.2, seed=3)
+    first = gradients(ctx, po, ncol, nrow, V, F[:nfaces])[0]
+    for _ in range(5):
+        assert np.array_equal(gradients(ctx, po, ncol, nrow, V, F[:nfaces])[0], first, equal_nan=True)

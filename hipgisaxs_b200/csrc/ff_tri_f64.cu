@@ -213,6 +213,7 @@ static int run_f64(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, const Rot
   const size_t part = sizeof(double) * NACC * (size_t)g->nqy;
   int nsplit = (int)std::max<long>(1, std::min<long>({(want + ctas - 1) / ctas, (long)tiles / 2, 32}));
   while (nsplit > 1 && nsplit * part > F64_PART_BYTES) --nsplit;
+  if (nsplit > 1 && is_capturing(st)) nsplit = 1;  // a captured call uses no workspace
   grid.z = nsplit;
   if (nsplit > 1) HGX_TRY(c->factors.reserve(nsplit * part));
   F64RowArgs a{sd, ntri, g->qx, g->qy, g->rowqz, g->nqy, g->nrow, g->ncol, F64_BLOCK / tpr, nsplit, R, out,

@@ -664,6 +664,12 @@ static int run(hgx_ctx c, hgx_qgrid g, const MmaTiles& t, const Rot9& R, void* o
   const size_t rec_bytes = (size_t)rows * t.ntiles * S::REC * 4;
   const size_t rec_pad = (rec_bytes + 255) & ~(size_t)255;
   const size_t part_bytes = nsplit > 1 ? (size_t)nsplit * rows * g->ncol * S::NACC * sizeof(double) : 0;
+  // nothing is allocated while the stream is captured (the FP32 kernel then takes the call), and a
+  // block that a graph holds stays allocated
+  if (is_capturing(st)) {
+    if (c->factors.bytes < b_bytes + rec_pad + part_bytes) return HGX_ERR_NO_MEMORY;
+    c->factors.captured = true;
+  }
   HGX_TRY(c->factors.reserve(b_bytes + rec_pad + part_bytes));
   unsigned char* base = reinterpret_cast<unsigned char*>(c->factors.p);
   HGX_CUDA(cudaFuncSetAttribute(ff_tri_mma_kernel<U, PAIRED, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,

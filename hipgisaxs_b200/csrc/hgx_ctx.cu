@@ -47,7 +47,15 @@ void* mapped_host_ptr(const void* p) {
 
 int DevBuf::reserve(size_t n) {
   if (n <= bytes) return HGX_OK;
-  release();
+  if (captured) {
+    kept.push_back(p);
+    p = nullptr;
+    bytes = 0;
+    captured = false;
+  }
+  if (p) cudaFree(p);
+  p = nullptr;
+  bytes = 0;
   size_t want = n < 4096 ? 4096 : n;
   cudaError_t e = cudaMalloc(&p, want);
   if (e != cudaSuccess) {
@@ -63,6 +71,18 @@ void DevBuf::release() {
   if (p) cudaFree(p);
   p = nullptr;
   bytes = 0;
+  for (void* k : kept) cudaFree(k);
+  kept.clear();
+  captured = false;
+}
+
+bool is_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream while another stream is captured
+    return false;
+  }
+  return cs != cudaStreamCaptureStatusNone;
 }
 
 // ------------------------------------------------------------- row table ----

@@ -46,10 +46,14 @@ void* mapped_host_ptr(const void* p);
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  bool captured = false;     // p is part of a captured graph: growing leaves it allocated until release
+  std::vector<void*> kept;   // such blocks
   int reserve(size_t n);  // grows (never shrinks); contents are not preserved
   void release();
   ~DevBuf() { release(); }
 };
+// The stream is being captured into a graph.
+bool is_capturing(cudaStream_t st);
 
 }  // namespace hgx
 
@@ -133,7 +137,7 @@ struct hgx_ctx_s {
   cudaStream_t stream = nullptr;
   unsigned* d_err = nullptr;  // device error word (DeviceError bits)
   hgx::DevBuf scratch;        // per-call scratch, grown on demand
-  hgx::DevBuf factors;        // row factors and partial sums of the tensor-core row kernel
+  hgx::DevBuf factors;        // row factors, partial sums and seed digits of the row-grid kernels
   hgx::DevBuf rowfc;          // per-row Fresnel coefficients on their way to the per-pixel layout
   hgx::TileView tiles;        // triangle tiles of the last FP32C form factor (in scratch)
   hgx::DevBuf staging;        // device copies of host inputs

@@ -90,9 +90,13 @@ int hgx_qgrid_destroy(hgx_qgrid g);
  * (include/ff/gpu/ff_num_gpu.cuh:55-58, src/ff/gpu/ff_tri_gpu.cu:395-521) and its CPU twin
  * NumericFormFactorC::compute_approx_triangle (src/ff/cpu/ff_tri_cpu.cpp:200-246).
  * shape_def: ntri x 8 doubles (s, nx, ny, nz, cx, cy, cz, pad) as read_shapes_file packs
- * them (src/ff/ff_num.cpp:1016-1030).  precision HGX_F64: FP64 throughout, one thread per
- * q-point (the plain form); HGX_F32C: FP32 phases and sums with compensated accumulation.
- * ff: nqz complex of type ff_type. */
+ * them (src/ff/ff_num.cpp:1016-1030).  precision HGX_F64: FP64 throughout (on
+ * detector rows factorised by row, else one thread per q-point); HGX_F32C: FP32 phases and sums with compensated accumulation.
+ * ff: nqz complex of type ff_type.
+ * With device arrays the call can be captured into a graph.  HGX_F64 then uses no memory of the
+ * context; HGX_F32C uses the context's tiles (make a call with these triangles before the capture, and
+ * no larger one while the graph is in use) and takes the tensor-core kernel only when an earlier call
+ * left room for its row factors, which then stay allocated until the context is destroyed. */
 int hgx_ff_triangles_q(hgx_ctx ctx, hgx_qgrid g, const double* shape_def, int ntri,
                        const double* rot9, int precision, void* ff, int ff_type);
 /* As hgx_ff_triangles_q with an explicit launch shape for the FP32 row kernel:

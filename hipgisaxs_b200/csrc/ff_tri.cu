@@ -1141,24 +1141,31 @@ static int prepare_tiles(hgx_ctx c, const double* sd, int ntri, const Rot9& R, b
   return HGX_OK;
 }
 
-// Which row kernel an untuned FP32C call takes.  Complex blocks: always the tensor cores (1.4 to 4.4 times
-// faster at every size tried).  Real blocks: the estimated times in us, from 712 sizes of 16 to 1024
-// columns, 60 to 2048 rows and 100 to 4,800 triangles.  A CTA of the FP32 kernel takes 21.5 per tile (however full)
-// and pixel per thread, CTAs that share an SM one after another as far as throughput goes; a CTA of
-// the tensor-core kernel (128 columns of a row, one per SM) 7.2 to start and to end, 1.5 more for each
-// further tile and 0.0108 per triangle.  So the FP32 kernel keeps single full tiles on large grids and, up
+// Which row kernel an untuned FP32C call takes: the estimated times in us.  A CTA of the FP32 kernel takes `fp32`
+// per tile (however full; with 1, 2 or 4 pixels per thread), CTAs that share an SM one after another as far as
+// throughput goes; a CTA of the tensor-core kernel (128 columns of a row, one per SM) `start` to start and to end,
+// `tile` more for each further tile and `tri` per triangle.  Paired real blocks from 712 sizes of 16 to 1024
+// columns, 60 to 2048 rows and 100 to 4,800 triangles, the others from 300 of 1 to 1500 columns, 1 to 60,000 rows
+// and 20 to 20,000 triangles.  Paired real blocks: the FP32 kernel keeps single full tiles on large grids and, up
 // to a few thousand triangles, grids of at most 64 columns (whose other half the tensor-core kernel pads)
 // with rows for about two CTAs per SM: 64 x 800 x 506 0.062 against 0.095 ms, 64 x 1024 x 1,000 0.133
 // / 0.178, 150 x 400 x 506 0.076 / 0.088.  On the other side 64 x 60 x 506 0.037 / 0.042, 128 x 300
-// x 506 0.074 / 0.082, 48 x 256 x 1,280 0.090 / 0.123, 130 x 512 x 4,800 0.52 / 0.90.  The margin leaves ties to
-// the tensor cores; over the 712 sizes the choice is at most 6% off the faster kernel where it
+// x 506 0.074 / 0.082, 48 x 256 x 1,280 0.090 / 0.123, 130 x 512 x 4,800 0.52 / 0.90.  One block (6 sums in
+// place of 12 or 24 to a phasor): 15 x 1,023 x 939 0.097 / 0.157, 48 x 600 x 300 0.048 / 0.064, on the other
+// side 57 x 300 x 711 0.072 / 0.074.  Four complex blocks: 1 x 1,006 x 383 0.106 / 0.114, else the tensor cores.
+// The margin leaves ties to the tensor cores; the choice is at most 11% off the faster kernel where it
 // takes the tensor cores and 10% where it takes the FP32 kernel.
 static bool rows_mma_pays(hgx_ctx c, hgx_qgrid g, int ntri) {
-  if (g->mode != 1) return true;
+  struct Model {
+    double fp32[3], start, tile, tri;
+  };
+  static const Model PAIRED = {{21.5, 43.0, 81.7}, 7.2, 1.5, 0.0108}, SINGLE = {{20.8, 27.5, 49.3}, 5.6, 0.3, 0.0136},
+                     FOUR = {{43.0, 75.0, 137.0}, 9.3, 2.2, 0.0140};
+  const Model& m = g->mode == 1 ? PAIRED : g->nk == 1 ? SINGLE : FOUR;
   const RowShape sh = row_shape(g->nrow, g->ncol, c->sm_count, 4);
   const double tiles = (ntri + TILE - 1) / TILE, sms = c->sm_count;
-  const double fp32 = ceil((double)sh.grid.x * sh.grid.y / sms) * tiles * 21.5 * (sh.P == 4 ? 3.8 : sh.P);
-  const double mma = ceil((double)g->nrow * ((g->ncol + 127) / 128) / sms) * (7.2 + 1.5 * (tiles - 1) + 0.0108 * ntri);
+  const double fp32 = ceil((double)sh.grid.x * sh.grid.y / sms) * tiles * m.fp32[sh.P >> 1];
+  const double mma = ceil((double)g->nrow * ((g->ncol + 127) / 128) / sms) * (m.start + m.tile * (tiles - 1) + m.tri * ntri);
   return !(fp32 < 0.9 * mma);
 }
 

@@ -192,6 +192,22 @@ static void launch_f64(const F64RowArgs& a, dim3 grid, cudaStream_t st) {
 
 constexpr size_t F64_PART_BYTES = (size_t)64 << 20;  // split partial sums
 
+// Whether the row kernel (P pixels per thread, `ctas` CTAs, `nsplit` ranges of triangles) is the faster one:
+// estimates per triangle in us, from 420 grids of 1 to 600 columns, 1 to 60,000 rows and 20 to 8,000 triangles.
+// A CTA's time on its SM does not depend on how many of its 32 or more columns are there, so grids of few columns
+// (scattered q-points count as rows of one) belong to ff_tri_f64_kernel, whose time goes with the q-points:
+// 1 x 60,000 x 5,000: 4.5 against 58.8 ms, single blocks 1.5 / 49.4; 8 x 18,502 x 1,896 4.5 / 7.1.
+// On the other side 16 x 24,746 x 1,253 6.9 / 6.2, 1 x 1,289 x 147 0.047 / 0.037.  Single blocks are
+// taken for real (complex ones cost the plain kernel 1.5 times as much).  The margin keeps the choice within 12%
+// of the plain kernel wherever it takes the row kernel.
+static bool rows_f64_pays(hgx_ctx c, hgx_qgrid g, int P, long ctas, int nsplit) {
+  const double sms = c->sm_count, load = (double)g->nqz / (128.0 * sms);
+  const bool complex4 = g->mode == 2 && g->nk == 4;
+  const double plain = complex4 ? std::max(0.295, 0.2 + 0.098 * load) : std::max(0.192, 0.13 + 0.067 * load);
+  const double cta = g->nk == 1 ? (P == 1 ? 0.066 : 0.097) : complex4 ? (P == 1 ? 0.115 : 0.166) : (P == 1 ? 0.075 : 0.115);
+  return !(plain < 1.15 * cta * std::max((double)ctas / sms, 1.3 / nsplit));
+}
+
 template <int U, bool PAIRED, typename OUT>
 static int run_f64(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, const Rot9& R, void* out) {
   constexpr int NACC = PAIRED ? 8 : 2 * U;
@@ -214,6 +230,7 @@ static int run_f64(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, const Rot
   int nsplit = (int)std::max<long>(1, std::min<long>({(want + ctas - 1) / ctas, (long)tiles / 2, 32}));
   while (nsplit > 1 && nsplit * part > F64_PART_BYTES) --nsplit;
   if (nsplit > 1 && is_capturing(st)) nsplit = 1;  // a captured call uses no workspace
+  if (!rows_f64_pays(c, g, P, ctas, nsplit)) return HGX_ERR_NO_MEMORY;
   grid.z = nsplit;
   if (nsplit > 1) HGX_TRY(c->factors.reserve(nsplit * part));
   F64RowArgs a{sd, ntri, g->qx, g->qy, g->rowqz, g->nqy, g->nrow, g->ncol, F64_BLOCK / tpr, nsplit, R, out,

@@ -23,7 +23,8 @@ struct MmaTiles {
 // Enqueues the form factor of a row grid (g->mode 1 or 2).
 int ff_rows_mma(hgx_ctx c, hgx_qgrid g, const MmaTiles& t, const Rot9& R, void* out, int ff_type);
 
-// The same in FP64.  HGX_ERR_NO_MEMORY: nothing was enqueued, the plain kernel takes the call.
+// The same in FP64.  HGX_ERR_NO_MEMORY: nothing was enqueued, the plain kernel takes the call (no room for the
+// split sums, or a grid on which it is the faster one).
 int ff_rows_f64(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, const Rot9& R, void* out, int ff_type);
 
 }  // namespace hgx

@@ -53,18 +53,27 @@ __device__ __forceinline__ cx<float> expi_turns_real<float>(double u) {
   return cx<float>{e.x, e.y};
 }
 template <typename T>
-__device__ __forceinline__ cx<T> expi_real(double ph) { return expi_turns_real<T>(ph * INV_2PI_R); }
+__device__ __forceinline__ cx<T> expi_real(double ph);
+template <>
+__device__ __forceinline__ cx<double> expi_real<double>(double ph) {
+  double s, c;
+  sincos_radians(ph, &s, &c);
+  return cx<double>{c, s};
+}
+template <>
+__device__ __forceinline__ cx<float> expi_real<float>(double ph) { return expi_turns_real<float>(ph * INV_2PI_R); }
 
-// a / b.  FP64: b's reciprocal by two Newton steps from the FP32 approximation (23 bits), without
-// the branches of the IEEE division; within two ulp for 1e-37 < |b| < 1e37
-// (sines and phases here).
+// a / b.  FP64: b's reciprocal by two Newton steps from the FP32 approximation (23 bits) and the quotient
+// corrected by its remainder, without the branches of the IEEE division; rounded as it is but for rare ties, for
+// 1e-37 < |b| < 1e37 (sines and phases here).
 __device__ __forceinline__ double quotient(double a, double b) {
   float y0;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"((float)b));
   double y = (double)y0;
   y = fma(y, fma(-b, y, 1.0), y);
   y = fma(y, fma(-b, y, 1.0), y);
-  return a * y;
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
 }
 __device__ __forceinline__ float quotient(float a, float b) { return __fdividef(a, b); }
 
@@ -176,8 +185,13 @@ static __device__ __noinline__ cx<T> box_axial_real(const Dist& Z, double qz) {
   return s;
 }
 
-// (sin x - x cos x) / x^3
+// (sin x - x cos x) / x^3, below 1/2 its series (the next term is below 3e-18)
 __device__ __forceinline__ double sphere_kernel(double x, double) {
+  if (x < 0.5) {
+    const double z = x * x;
+    return 1. / 3. - z * (1. / 30. - z * (1. / 840. - z * (1. / 45360. - z * (1. / 3991680. -
+                     z * (1. / 518918400. - z * (1. / 93405312000.))))));
+  }
   const cx<double> e = expi_real<double>(x);
   return (e.y - x * e.x) / (x * x * x);
 }

@@ -77,14 +77,10 @@ __device__ __forceinline__ float sin_half_turn(float x) {
   return p * x;
 }
 
-// sin and cos of 2 pi u in FP64: u reduced exactly to r in [-1/8, 1/8] turn by the nearest quarter
-// (adding 1.5 2^52 leaves it in the low mantissa bits), then sin(2 pi r) / r and (cos(2 pi r) - 1) / r^2 as polynomials
-// of degree 6 in r^2 (Chebyshev fits over the interval; both within 1.4e-16 of the value).  18 FP64
-// operations.  Valid for |u| < 2^50; NaN and infinite u give NaN.
-__device__ __forceinline__ void sincos_turns(double u, double* s, double* c) {
-  const double t = fma(u, 4.0, RND52);
-  const int k = __double2loint(t);
-  const double r = fma(t - RND52, -0.25, u), z = r * r;
+// sin and cos of 2 pi (r + k/4), |r| <= 1/8: sin(2 pi r) / r and (cos(2 pi r) - 1) / r^2 as polynomials of
+// degree 6 in r^2 (Chebyshev fits over the interval; both within 1.4e-16 of the value), k's quarter turns.
+__device__ __forceinline__ void sincos_quarters(double r, int k, double* s, double* c) {
+  const double z = r * r;
   double p = 3.780830078125, q = -1.698876953125;
   p = fma(p, z, -15.093802528381348);
   q = fma(q, z, 7.9031996917724605);
@@ -104,6 +100,19 @@ __device__ __forceinline__ void sincos_turns(double u, double* s, double* c) {
   const double a = odd ? q : p, b = odd ? p : q;
   *s = __hiloint2double(__double2hiint(a) ^ ((k & 2) << 30), __double2loint(a));
   *c = __hiloint2double(__double2hiint(b) ^ (((k + 1) & 2) << 30), __double2loint(b));
+}
+// sin and cos of 2 pi u in FP64: u reduced exactly by the nearest quarter turn (adding 1.5 2^52 leaves it in
+// the low mantissa bits).  18 FP64 operations.  Valid for |u| < 2^50; NaN and infinite u give NaN.
+__device__ __forceinline__ void sincos_turns(double u, double* s, double* c) {
+  const double t = fma(u, 4.0, RND52);
+  sincos_quarters(fma(t - RND52, -0.25, u), __double2loint(t), s, c);
+}
+// sin and cos of x radians: the turns x / 2 pi less the nearest quarter by multiply-adds with both parts of
+// 1 / 2 pi, so that the reduced angle has no error but its own rounding.  20 FP64 operations.
+__device__ __forceinline__ void sincos_radians(double x, double* s, double* c) {
+  const double hi = 0.15915494309189535, lo = -9.839338337591243e-18;  // 1 / 2 pi
+  const double t = fma(x, 4.0 * hi, RND52);
+  sincos_quarters(fma(x, lo, fma(x, hi, -0.25 * (t - RND52))), __double2loint(t), s, c);
 }
 
 // sin of 2 pi r for |r| <= 1/4 (a polynomial of degree 8 in r^2 times r, a Chebyshev fit; within

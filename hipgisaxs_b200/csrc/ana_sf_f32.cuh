@@ -1,6 +1,11 @@
-// FP32-compensated pieces of the analytic form factors for a real rotated q (grids whose DWBA qz
-// blocks are real: a vacuum particle layer): every phase formed and range-reduced in FP64, only the
-// transcendental of the reduced argument and the sums in FP32.
+// FP32-compensated bodies of the analytic form factors and the lattice structure factor for a
+// real rotated q (grids whose DWBA qz blocks are real: a vacuum particle layer): every phase
+// formed and range-reduced in FP64, only the transcendental of the reduced argument and the sums in
+// FP32.  They serve grain_dwba_f32c_kernel and ff_analytic_f32c_kernel, one thread per (pixel,
+// block); ana_sf_real.cuh has the bodies of the kernels with one thread per pixel.
+//
+// Lattice structure factor (src/sf/sf.cpp:164-246): see ana_sf_real.cuh; N is returned where
+// the reference's guard |1 - e| <= eps takes N.
 #pragma once
 
 #include "ana_sf.cuh"
@@ -33,6 +38,12 @@ __device__ __forceinline__ float sinc_from(double x, float sinx) {
   if (fabs(x) > 1e-2) return sinx / (float)x;
   const float x2 = (float)(x * x);
   return 1.f - x2 * (1.f / 6.f - x2 * (1.f / 120.f));
+}
+
+// with_phase of ana_sf.cuh: v e^{i m.tv}, not evaluated at the origin
+__device__ __forceinline__ cf with_phase_f(cf v, const double* m, const double* tv) {
+  if (tv[0] == 0.0 && tv[1] == 0.0 && tv[2] == 0.0) return v;
+  return cmul(v, expi_f(m[0] * tv[0] + m[1] * tv[1] + m[2] * tv[2]));
 }
 
 // an integer-valued k (|k| < 2^51) is odd
@@ -99,6 +110,163 @@ __device__ __forceinline__ float sphere_kernel_f(double x) {
   }
   const cf e = expi_f(x);
   return (e.y - (float)x * e.x) / (float)(x * x * x);
+}
+
+// The analytic form factor of shape `a` (SHAPE: cylinder, sphere or box) at the real rotated
+// q (m) translated by tv: ff_analytic_eval of ana_sf.cuh in FP32C.
+template <int SHAPE>
+__device__ __forceinline__ cf ff_analytic_f32c(const AnaShape& a, const double* m, const double* tv) {
+  const Dist& X = a.d[0];
+  const Dist& Y = a.d[1];
+  const Dist& Z = a.d[2];
+  cf out{0.f, 0.f};
+  if (SHAPE == SH_CYLINDER) {  // ff_ana_cylinder.cpp:34-42,100-117 (unweighted)
+    const double qpar = sqrt(m[0] * m[0] + m[1] * m[1]);
+    float fr = 0.f;
+    for (int i = 0; i < X.n; ++i) {
+      const double r = X.v[i], x = qpar * r;
+      if (x * x > CUTINY_REF) fr += (float)(2. * PI_REF * r * r) * (j1f((float)x) / (float)x);
+    }
+    const cf gh = cyl_height_sum_f32(Z, m[2]);
+    out = with_phase_f(cscale(gh, fr), m, tv);
+  } else if (SHAPE == SH_SPHERE) {  // ff_ana_sphere.cpp:33-45,95-107 (weighted)
+    const double q = sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+    cf acc{0.f, 0.f};
+    if (q >= 2.2250738585072014e-308)
+      for (int i = 0; i < X.n; ++i) {
+        const double R = X.v[i];
+        const float c0 = sphere_kernel_f(q * R) * (float)(4. * PI_REF * R * R * R * X.w[i]);
+        acc = cadd(acc, cscale(expi_f(m[2] * R), c0));
+      }
+    out = with_phase_f(acc, m, tv);
+  } else if (SHAPE == SH_BOX) {  // ff_ana_box.cpp:35-42,96-125 (weighted)
+    float sx = 0.f, sy = 0.f;
+    cf sz{0.f, 0.f};
+    for (int i = 0; i < X.n; ++i) {
+      const double x = m[0] * 0.5 * X.v[i];
+      sx += sinc_from(x, expi_f(x).y) * (float)(X.v[i] * X.w[i]);
+    }
+    for (int i = 0; i < Y.n; ++i) {
+      const double x = m[1] * 0.5 * Y.v[i];
+      sy += sinc_from(x, expi_f(x).y) * (float)(Y.v[i] * Y.w[i]);
+    }
+    for (int i = 0; i < Z.n; ++i) {
+      const double x = m[2] * 0.5 * Z.v[i];
+      const cf e = expi_f(x);
+      sz = cadd(sz, cscale(e, sinc_from(x, e.y) * (float)(Z.v[i] * Z.w[i])));
+    }
+    out = with_phase_f(cscale(sz, sx * sy), m, tv);
+  }
+  return out;
+}
+
+// The quad of four lanes (one per DWBA block) of the fused grain kernel: the sum of v over the
+// quad, the same bits in every lane (an xor butterfly of commutative adds).
+__device__ __forceinline__ float quad_sum(float v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  return v;
+}
+
+// ff_analytic_f32c for a quad whose rotated in-plane q (m[0], m[1]) is the same in its four
+// lanes (the element's rotation keeps qz out of them): what depends on the in-plane q only - the
+// cylinder's radial sum, the box's x and y sums - is split among the lanes (lane k takes the
+// samples k, k + 4, ...) and summed by quad_sum; the qz parts stay per lane.  Every lane of the
+// warp calls it (shuffles); the sphere, whose |q| involves qz, keeps ff_analytic_f32c.
+template <int SHAPE>
+__device__ __forceinline__ cf ff_analytic_f32c_quad(const AnaShape& a, const double* m, const double* tv, int k) {
+  const Dist& X = a.d[0];
+  const Dist& Y = a.d[1];
+  const Dist& Z = a.d[2];
+  if (SHAPE == SH_CYLINDER) {
+    const double qpar = sqrt(m[0] * m[0] + m[1] * m[1]);
+    float fr = 0.f;
+    for (int i = k; i < X.n; i += 4) {
+      const double r = X.v[i], x = qpar * r;
+      if (x * x > CUTINY_REF) fr += (float)(2. * PI_REF * r * r) * (j1f((float)x) / (float)x);
+    }
+    fr = quad_sum(fr);
+    const cf gh = cyl_height_sum_f32(Z, m[2]);
+    return with_phase_f(cscale(gh, fr), m, tv);
+  } else if (SHAPE == SH_BOX) {
+    float sx = 0.f, sy = 0.f;
+    for (int i = k; i < X.n; i += 4) {
+      const double x = m[0] * 0.5 * X.v[i];
+      sx += sinc_from(x, expi_f(x).y) * (float)(X.v[i] * X.w[i]);
+    }
+    for (int i = k; i < Y.n; i += 4) {
+      const double x = m[1] * 0.5 * Y.v[i];
+      sy += sinc_from(x, expi_f(x).y) * (float)(Y.v[i] * Y.w[i]);
+    }
+    sx = quad_sum(sx);
+    sy = quad_sum(sy);
+    cf sz{0.f, 0.f};
+    for (int i = 0; i < Z.n; ++i) {
+      const double x = m[2] * 0.5 * Z.v[i];
+      const cf e = expi_f(x);
+      sz = cadd(sz, cscale(e, sinc_from(x, e.y) * (float)(Z.v[i] * Z.w[i])));
+    }
+    return with_phase_f(cscale(sz, sx * sy), m, tv);
+  }
+  return ff_analytic_f32c<SHAPE>(a, m, tv);
+}
+
+// sin(N theta_r / 2) / sin(theta_r / 2) on the principal angle theta_r of e^{i theta}
+__device__ __forceinline__ float dirichlet_principal(double theta, double N) {
+  if (N == 1.0) return 1.f;
+  double t = theta * INV_2PI_A;
+  t -= round_fp64(t);
+  if (t == 0.0) return (float)N;
+  double v = N * t;
+  const double k = round_fp64(v);
+  v -= k;
+  const float num = odd_integer(k) ? -sinpi_f32((float)v) : sinpi_f32((float)v);
+  return num / sinpi_f32((float)t);
+}
+
+// the b-axis factor: e^{i pi k (N - 1)} sin(N theta / 2) / sin(theta / 2)
+__device__ __forceinline__ cf dirichlet_b(double theta, double N) {
+  if (N == round_fp64(N)) return cf{dirichlet_principal(theta, N), 0.f};
+  const double u = theta * INV_2PI_A;
+  const double k = round_fp64(u), t = u - k;
+  if (t == 0.0) return cf{(float)N, 0.f};
+  double v = N * u;
+  const double kv = round_fp64(v);
+  v -= kv;
+  const float num = odd_integer(kv) ? -sinpi_f32((float)v) : sinpi_f32((float)v);
+  const float den = odd_integer(k) ? -sinpi_f32((float)t) : sinpi_f32((float)t);
+  return cscale(expi_turns(k * (N - 1.0) * 0.5), num / den);
+}
+
+// sf_lattice_eval of ana_sf.cuh for a real rotated q, FP32C.  The b angle keeps the
+// reference's lb[2] * lb[2] term (src/sf/sf.cpp:212).
+__device__ __forceinline__ cf sf_lattice_f32c(const SfLat& L, const double* m) {
+  const double ta = m[0] * L.la[0] + m[1] * L.la[1] + m[2] * L.la[2];
+  const double tb = m[0] * L.lb[0] + m[1] * L.lb[1] + L.lb[2] * L.lb[2];
+  const double tc = m[0] * L.lc[0] + m[1] * L.lc[1] + m[2] * L.lc[2];
+  const float sa = dirichlet_principal(ta, L.rep[0]);
+  const cf sb = dirichlet_b(tb, L.rep[1]);
+  const float sc = dirichlet_principal(tc, L.rep[2]);
+  const cf t3 = expi_f(m[0] * L.center[0] + m[1] * L.center[1] + m[2] * L.center[2]);
+  return cmul(t3, cscale(sb, sa * sc));
+}
+
+// sf_lattice_f32c for a quad whose rotated in-plane q is the same in its four lanes, with an
+// in-plane a vector and an integer b repetition: the a- and b-axis factors do not depend on
+// the block, so the even lanes evaluate the a factor and the odd lanes the b factor (the same
+// code on other arguments) and a shuffle exchanges them; the c factor and the centre phase
+// stay per lane.  Every lane of the warp calls it.
+__device__ __forceinline__ cf sf_lattice_f32c_paired(const SfLat& L, const double* m, int k) {
+  const bool odd = (k & 1) != 0;
+  const double th = odd ? m[0] * L.lb[0] + m[1] * L.lb[1] + L.lb[2] * L.lb[2]
+                        : m[0] * L.la[0] + m[1] * L.la[1] + m[2] * L.la[2];
+  const float own = dirichlet_principal(th, odd ? L.rep[1] : L.rep[0]);
+  const float other = __shfl_xor_sync(0xffffffffu, own, 1);
+  const float sa = odd ? other : own, sb = odd ? own : other;
+  const double tc = m[0] * L.lc[0] + m[1] * L.lc[1] + m[2] * L.lc[2];
+  const float sc = dirichlet_principal(tc, L.rep[2]);
+  const cf t3 = expi_f(m[0] * L.center[0] + m[1] * L.center[1] + m[2] * L.center[2]);
+  return cscale(t3, sb * sa * sc);
 }
 
 }  // namespace hgx

@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "ana_sf.cuh"
+#include "ana_sf_f32.cuh"
 #include "ana_sf_real.cuh"
 #include "cplx.cuh"
 #include "hgx_internal.cuh"
@@ -85,12 +86,36 @@ __global__ void __launch_bounds__(128) ff_analytic_real_kernel(const AnaArgs* __
   }
 }
 
+// FP32C on the same grids with one thread per q-point (ana_sf_f32.cuh), where the blocks share nothing or
+// the pixels are too few.
+template <int SHAPE, typename OUT>
+__global__ void __launch_bounds__(128) ff_analytic_f32c_kernel(const AnaArgs* __restrict__ ap) {
+  const AnaArgs& a = *ap;
+  long iz = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (iz >= a.nqz) return;
+  long iy = iz % a.nqy;
+  const double qx = a.qx[iy], qy = a.qy[iy], qz = a.qz[iz].x;
+  double m[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) m[j] = a.R.r[3 * j] * qx + a.R.r[3 * j + 1] * qy + a.R.r[3 * j + 2] * qz;
+  const cf v = ff_analytic_f32c<SHAPE>(a.s, m, a.tv);
+  put<OUT>(a.out, iz, zd((double)v.x, (double)v.y));
+}
+
 template <typename T, typename OUT>
 static void launch_real(int shape, long n, cudaStream_t st, const AnaArgs* d_args) {
   const unsigned blocks = (unsigned)((n + 127) / 128);
   if (shape == SH_CYLINDER) ff_analytic_real_kernel<T, SH_CYLINDER, OUT><<<blocks, 128, 0, st>>>(d_args);
   else if (shape == SH_SPHERE) ff_analytic_real_kernel<T, SH_SPHERE, OUT><<<blocks, 128, 0, st>>>(d_args);
   else ff_analytic_real_kernel<T, SH_BOX, OUT><<<blocks, 128, 0, st>>>(d_args);
+}
+
+template <typename OUT>
+static void launch_points(int shape, long n, cudaStream_t st, const AnaArgs* d_args) {
+  const unsigned blocks = (unsigned)((n + 127) / 128);
+  if (shape == SH_CYLINDER) ff_analytic_f32c_kernel<SH_CYLINDER, OUT><<<blocks, 128, 0, st>>>(d_args);
+  else if (shape == SH_SPHERE) ff_analytic_f32c_kernel<SH_SPHERE, OUT><<<blocks, 128, 0, st>>>(d_args);
+  else ff_analytic_f32c_kernel<SH_BOX, OUT><<<blocks, 128, 0, st>>>(d_args);
 }
 
 // ------------------------------------------------------------------- host side ----
@@ -254,9 +279,16 @@ int ff_analytic_launch(hgx_ctx c, hgx_qgrid g, const AnaArgs& host_args, void* o
   HGX_CUDA(cudaMemcpyAsync(d_args, &a, sizeof(AnaArgs), cudaMemcpyHostToDevice, c->stream));
   dim3 grid((g->nqz + 127) / 128);
   const int sh = a.s.shape;
-  if (g->mode == 1 && (sh == SH_CYLINDER || sh == SH_SPHERE || sh == SH_BOX)) {
-    const bool f = precision == HGX_F32C;
-    if (f && a.out_c64) launch_real<float, float2>(sh, g->nqy, c->stream, d_args);
+  // Real qz: a thread per pixel where the blocks share the in-plane sums and the pixels fill the GPU.  FP32C else takes
+  // a thread per q-point (15 samples, us, pixels / q-points: 128 x 96 flat boxes 28 / 20, 300 x 200 tilted cylinders 34
+  // / 26, 640 x 481 spheres 88 / 76; on the other side 300 x 200 flat cylinders 21 / 26), FP64 only for few
+  // tilted cylinders, in the complex form (40 x 28: 61 / 41; 300 x 200 tilted 61 / 94).
+  const bool flat = a.R.r[2] == 0.0 && a.R.r[5] == 0.0, few = g->nqy < 30000, f = precision == HGX_F32C;
+  const bool points = f ? !flat || sh == SH_SPHERE || few : sh == SH_CYLINDER && !flat && few && a.s.d[0].n > 1;
+  if (g->mode == 1 && (sh == SH_CYLINDER || sh == SH_SPHERE || sh == SH_BOX) && (f || !points)) {
+    if (points && a.out_c64) launch_points<float2>(sh, g->nqz, c->stream, d_args);
+    else if (points) launch_points<double2>(sh, g->nqz, c->stream, d_args);
+    else if (f && a.out_c64) launch_real<float, float2>(sh, g->nqy, c->stream, d_args);
     else if (f) launch_real<float, double2>(sh, g->nqy, c->stream, d_args);
     else if (a.out_c64) launch_real<double, float2>(sh, g->nqy, c->stream, d_args);
     else launch_real<double, double2>(sh, g->nqy, c->stream, d_args);

@@ -438,6 +438,89 @@ __global__ void __launch_bounds__(128, 4) grain_dwba_real_kernel(FusedArgs a) {
   if (live) out[i] = acc;
 }
 
+// The same in FP32C with four threads per pixel, one per block: the quad layout and order of sums of
+// grain_dwba_kernel, the form and structure factors from ana_sf_f32.cuh, the DWBA terms in FP32 and
+// the intensity accumulated in FP64.  For images of too few pixels for one thread each, and for
+// form factors of several samples that neither the blocks nor the grains share (grain_real_plan).
+// SPLIT: the grains are split over grid z (an instance of its own: the split costs the other registers and 5%).
+template <int SHAPE, bool SPLIT>
+__global__ void __launch_bounds__(128) grain_dwba_f32c_kernel(FusedArgs a) {
+  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long i = t >> 2;
+  const int k = (int)(t & 3);
+  const bool live = i < a.n;  // every lane takes part in the shuffles
+  const long ii = live ? i : 0;
+  const double qx = a.qx[ii], qy = a.qy[ii];
+  const double qz = a.qz[k * a.n + ii].x;
+  const double2 fcd = a.fc[k * a.n + ii];
+  const cf fc{(float)fcd.x, (float)fcd.y};
+  const int base = (threadIdx.x & 31) & ~3;
+  const long cy = blockIdx.y;  // the candidate of a population launch
+  const AnaShape* shapes = a.shapes + cy * a.ps_shape;
+  const FusedElem* elems = a.elems + cy * a.ps_elem;
+  const double* grains = a.grains + cy * a.ps_grain;
+  const double* elem_rot = a.elem_rot + cy * a.ps_er;
+  const ScaleEntry* scales = a.scales + cy * a.ps_scale;
+  int ga = a.g0, gb = a.g1;
+  double* out = a.out + cy * a.ps_out;
+  if (SPLIT) {
+    gb = a.g0 + (int)((long)(blockIdx.z + 1) * (a.g1 - a.g0) / gridDim.z);
+    ga = a.g0 + (int)((long)blockIdx.z * (a.g1 - a.g0) / gridDim.z);
+    out = a.part + (long)blockIdx.z * a.n;
+  }
+  double acc = (!SPLIT && live && k == 0) ? out[i] : 0.0;
+  for (int g = ga; g < gb; ++g) {
+    const double* gp = grains + 12 * (long)g;
+    cf ff{0.f, 0.f};
+    for (int e = 0; e < a.nelem; ++e) {
+      const double* er = elem_rot + 9 * ((long)g * a.nelem + e);
+      double m[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) m[j] = er[3 * j] * qx + er[3 * j + 1] * qy + er[3 * j + 2] * qz;
+      // the same grain and element in every lane of the warp: the test is warp-uniform; the
+      // split pays when the in-plane sums have four samples or more
+      const cf eff = (er[2] == 0.0 && er[5] == 0.0 && shapes[e].d[0].n >= 4)
+                         ? ff_analytic_f32c_quad<SHAPE>(shapes[e], m, elems[e].loc, k)
+                         : ff_analytic_f32c<SHAPE>(shapes[e], m, elems[e].loc);
+      ff = cadd(ff, cmul(cf{(float)elems[e].dre, (float)elems[e].dim}, eff));
+    }
+    double mr[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) mr[j] = gp[3 * j] * qx + gp[3 * j + 1] * qy + gp[3 * j + 2] * qz;
+    const ScaleEntry* sp = scales + (long)g * a.nscale;
+    const bool flat = gp[2] == 0.0 && gp[5] == 0.0;  // the grain rotation keeps qz out of mr[0], mr[1]
+    for (int si = 0; si < a.nscale; ++si) {
+      cf sfv;
+      if (a.sfbuf) {
+        const double2 v = a.sfbuf[k * a.n + ii];
+        sfv = cf{(float)v.x, (float)v.y};
+      } else {
+        SfLat L;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          L.la[d] = sp[si].la[d];
+          L.lb[d] = sp[si].lb[d];
+          L.lc[d] = sp[si].lc[d];
+          L.rep[d] = sp[si].rep[d];
+          L.center[d] = gp[9 + d];
+        }
+        // warp-uniform: the same grain and sample in every lane
+        sfv = (flat && L.la[2] == 0.0 && L.rep[1] == round_fp64(L.rep[1])) ? sf_lattice_f32c_paired(L, mr, k)
+                                                                           : sf_lattice_f32c(L, mr);
+      }
+      const cf term = cmul(cmul(fc, sfv), ff);
+      cf sum{0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        sum = cadd(sum, cf{__shfl_sync(0xffffffffu, term.x, base + j),
+                           __shfl_sync(0xffffffffu, term.y, base + j)});
+      const float w = (float)sp[si].w;
+      acc += (double)(w * w * (sum.x * sum.x + sum.y * sum.y));
+    }
+  }
+  if (live && k == 0) out[i] = acc;
+}
+
 // out += the splits' sums, in order.
 __global__ void grain_sum_kernel(const double* __restrict__ part, int splits, long n, double* __restrict__ out) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -452,13 +535,68 @@ static bool grain_real_shape(int shape) {
   return shape == SH_CYLINDER || shape == SH_SPHERE || shape == SH_BOX;
 }
 
+// The kernels of a structure on real qz (grain_real_plan).
+enum GrainKernel { GRAIN_PIXEL, GRAIN_QUAD, GRAIN_COMPLEX };
+
 template <typename T>
-static void launch_grain_real(int shape, dim3 grid, cudaStream_t st, const FusedArgs& a) {
+static void launch_grain_pixel(int shape, dim3 grid, cudaStream_t st, const FusedArgs& a) {
   switch (shape) {
     case SH_CYLINDER: grain_dwba_real_kernel<T, SH_CYLINDER><<<grid, 128, 0, st>>>(a); break;
     case SH_SPHERE: grain_dwba_real_kernel<T, SH_SPHERE><<<grid, 128, 0, st>>>(a); break;
     default: grain_dwba_real_kernel<T, SH_BOX><<<grid, 128, 0, st>>>(a); break;
   }
+}
+static unsigned grain_real_ctas(GrainKernel k, long n) { return (unsigned)(((k == GRAIN_QUAD ? 4 * n : n) + 127) / 128); }
+static void launch_grain_real(GrainKernel k, int shape, bool f32c, dim3 grid, cudaStream_t st, const FusedArgs& a) {
+  if (k == GRAIN_PIXEL) {
+    if (f32c) launch_grain_pixel<float>(shape, grid, st, a);
+    else launch_grain_pixel<double>(shape, grid, st, a);
+    return;
+  }
+  const bool split = grid.z > 1;
+#define HGX_QUAD_LAUNCH(S)                                                    \
+  (split ? (void)(grain_dwba_f32c_kernel<S, true><<<grid, 128, 0, st>>>(a)) \
+         : (void)(grain_dwba_f32c_kernel<S, false><<<grid, 128, 0, st>>>(a)))
+  switch (shape) {
+    case SH_CYLINDER: HGX_QUAD_LAUNCH(SH_CYLINDER); break;
+    case SH_SPHERE: HGX_QUAD_LAUNCH(SH_SPHERE); break;
+    default: HGX_QUAD_LAUNCH(SH_BOX); break;
+  }
+#undef HGX_QUAD_LAUNCH
+}
+
+// Which kernel a structure on real qz takes.  npix: pixels of a launch; samples: the largest number of samples of
+// a dimension; flat: no rotation takes qz into the rotated in-plane q and no a vector has a z component.
+// FP32C: a thread per pixel shares the in-plane sums among the blocks of flat grains and keeps the form factors
+// of successive ones; where there is nothing to share (tilted grains, boxes of several samples, one grain of
+// spheres) or too few pixels the quad kernel is the faster one.  Times in ms, pixel / quad kernel: 257 x 200 x
+// 9 tilted grains of boxes of 11 samples 0.275 / 0.193, of cylinders 0.188 / 0.148; 100 x 80 x 2 tilted boxes 0.073 /
+// 0.036; 40 x 28, one flat grain of cylinders 0.031 / 0.025; on the other side 600 x 300 x 60 flat grains of
+// cylinders 0.102 / 0.84, of boxes of one sample 0.59 / 0.91, tilted ones of spheres 0.73 / 0.88.
+// FP64: a few tilted grains of cylinders on few pixels go to the complex kernel's four threads per pixel (40 x 28,
+// 11 samples: 0.061 / 0.049).
+static GrainKernel grain_real_plan(int shape, bool f32c, int samples, bool flat, long npix, int ngrains) {
+  const bool few = npix < 40000, single = samples <= 2;
+  if (!f32c) return shape == SH_CYLINDER && !flat && !single && npix < 6000 && ngrains <= 4 ? GRAIN_COMPLEX : GRAIN_PIXEL;
+  if (!flat) return shape == SH_BOX || !single || (few && ngrains < 32) ? GRAIN_QUAD : GRAIN_PIXEL;
+  if (shape == SH_BOX) return !single || (few && ngrains <= 2) ? GRAIN_QUAD : GRAIN_PIXEL;
+  return (few && ngrains <= 2) || (shape == SH_SPHERE && !single && ngrains == 1) ? GRAIN_QUAD : GRAIN_PIXEL;
+}
+
+static int grain_samples(const std::vector<AnaShape>& shapes) {
+  int n = 1;
+  for (const AnaShape& s : shapes)
+    for (const Dist& d : s.d) n = std::max(n, d.n);
+  return n;
+}
+static bool grains_flat(const std::vector<double>& gt, const std::vector<double>& er, const std::vector<ScaleEntry>& plan) {
+  for (size_t i = 0; i < gt.size(); i += 12)
+    if (gt[i + 2] != 0.0 || gt[i + 5] != 0.0) return false;
+  for (size_t i = 0; i < er.size(); i += 9)
+    if (er[i + 2] != 0.0 || er[i + 5] != 0.0) return false;
+  for (const ScaleEntry& e : plan)
+    if (e.la[2] != 0.0) return false;
+  return true;
 }
 
 // The tangent of the fused grain loop (FP64, real qz): for one direction of the fit
@@ -1036,10 +1174,14 @@ static int fused_structure(hgx_ctx c, hgx_qgrid g, HigWork& w, const hig::Struct
   for (int e = 1; e < nelem; ++e)
     if (shapes[e].shape != one) one = 0;
   // grids with real qz blocks (paired rows) and one shape with a real-qz body
-  if (g->mode == 1 && grain_real_shape(one)) {
-    const unsigned blocks1 = (unsigned)((a.n + 127) / 128);
-    // four CTAs of 128 threads run per SM; grains are split where the pixels do not fill them
-    const int splits = (int)std::max<long>(1, std::min<long>({4L * c->sm_count / blocks1, (long)ngr / 4, 32}));
+  const bool real = g->mode == 1 && grain_real_shape(one), f32c = precision == HGX_F32C;
+  const GrainKernel plan_k = real ? grain_real_plan(one, f32c, grain_samples(shapes), grains_flat(gt, er, plan), a.n, ngr)
+                                  : GRAIN_COMPLEX;
+  if (plan_k != GRAIN_COMPLEX) {
+    const unsigned ctas = grain_real_ctas(plan_k, a.n);
+    // four CTAs of 128 threads run per SM (nine of the quad kernel); grains are split where the pixels do not fill them
+    const int splits = (int)std::max<long>(
+        1, std::min<long>({(plan_k == GRAIN_QUAD ? 9L : 4L) * c->sm_count / ctas, (long)ngr / 4, 32}));
     if (splits > 1) {
       HGX_TRY(w.gpart.reserve(sizeof(double) * a.n * splits));
       a.part = (double*)w.gpart.p;
@@ -1047,8 +1189,7 @@ static int fused_structure(hgx_ctx c, hgx_qgrid g, HigWork& w, const hig::Struct
     for (int g0 = 0; g0 < ngr; g0 += REAL_GRAINS_PER_LAUNCH) {
       a.g0 = g0;
       a.g1 = std::min(ngr, g0 + REAL_GRAINS_PER_LAUNCH);
-      if (precision == HGX_F32C) launch_grain_real<float>(one, dim3(blocks1, 1, splits), st, a);
-      else launch_grain_real<double>(one, dim3(blocks1, 1, splits), st, a);
+      launch_grain_real(plan_k, one, f32c, dim3(ctas, 1, splits), st, a);
       if (splits > 1) grain_sum_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a.part, splits, a.n, a.out);
       HGX_CUDA(cudaGetLastError());
     }
@@ -1656,7 +1797,7 @@ namespace {
 struct PopStruct {
   int ngr = 0, nscale = 0, nelem = 0, shape = 0;
   bool liquid = false;
-  bool real = false, f32c = false;  // grain_dwba_real_kernel, its precision
+  bool real = false, f32c = false;  // real qz and one shape with a real-qz body; the precision
   // byte offsets in the staging block of each table's region; a region holds the table of every
   // candidate in turn (candidate i at i x the table's size)
   size_t o_shapes = 0, o_elems = 0, o_gt = 0, o_er = 0, o_sc = 0;
@@ -1772,12 +1913,12 @@ int pop_enqueue(hgx_hig_pop_s& P, cudaStream_t st) {
     for (int g0 = 0; g0 < ps.ngr; g0 += chunk) {
       a.g0 = g0;
       a.g1 = std::min(ps.ngr, g0 + chunk);
-      if (ps.real) {
-        const dim3 g1((unsigned)((n + 127) / 128), (unsigned)P.npop);
-        if (ps.f32c) launch_grain_real<float>(ps.shape, g1, st, a);
-        else launch_grain_real<double>(ps.shape, g1, st, a);
+      const int variant = P.variants[vi++];  // a GrainKernel other than GRAIN_COMPLEX, or -1 - (paired)
+      if (variant >= 0) {
+        const GrainKernel gk = (GrainKernel)variant;
+        launch_grain_real(gk, ps.shape, ps.f32c, dim3(grain_real_ctas(gk, n), (unsigned)P.npop), st, a);
       } else {
-        const int paired = P.variants[vi++];
+        const int paired = variant == -2;
 #define HGX_POP_LAUNCH(S)                                                   \
   (paired ? (void)(grain_dwba_kernel<S, 1><<<grid, 128, 0, st>>>(a))      \
           : (void)(grain_dwba_kernel<S, 0><<<grid, 128, 0, st>>>(a)))
@@ -1998,8 +2139,14 @@ int hgx_hig_population_eval(hgx_hig_pop p, const double* X, int nx, double* dist
   const int chunk = pop_chunk(p->npop);
   for (int k = 0; k < p->nstruct; ++k) {
     const PopStruct& ps = p->st[k];
-    if (ps.real) continue;
-    for (int g0 = 0; g0 < ps.ngr; g0 += chunk) v.push_back(pop_paired(all, k, g0, std::min(ps.ngr, g0 + chunk)));
+    GrainKernel gk = GRAIN_COMPLEX;
+    if (ps.real) {
+      bool flat = true;
+      for (const auto& T : all) flat = flat && grains_flat(T[k].f.gt, T[k].f.er, T[k].plan);
+      gk = grain_real_plan(ps.shape, ps.f32c, grain_samples(all[0][k].f.shapes), flat, p->n * p->npop, ps.ngr);
+    }
+    for (int g0 = 0; g0 < ps.ngr; g0 += chunk)
+      v.push_back(gk != GRAIN_COMPLEX ? (int)gk : -1 - (int)pop_paired(all, k, g0, std::min(ps.ngr, g0 + chunk)));
   }
   if (p->exec && v != p->variants) {  // another kernel variant: record the graph again
     cudaGraphExecDestroy(p->exec);

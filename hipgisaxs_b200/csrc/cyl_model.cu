@@ -191,6 +191,7 @@ __device__ __forceinline__ void cyl_rows_body(const CylCand& c, int bx, const do
                                               const double2* __restrict__ rowfc, RowTab* __restrict__ tab) {
   constexpr int L = CYL_ROW_LANES;
   const int row = (int)((bx * blockDim.x + threadIdx.x) / (2 * L)), lr = min(row, c.nrows - 1);
+  if (row - (int)(threadIdx.x & 31) / (2 * L) >= c.nrows) return;  // whole warps past the region's last row
   const int lane = threadIdx.x & (2 * L - 1), k = lane / L * 2;
   const int grow = c.row0 + lr;
   const double qz = rowqz[4L * grow + k].x;
@@ -338,18 +339,18 @@ __device__ __forceinline__ int warp_slot() {  // lanes 0, 8, 4, 16, 24 hold v[0]
   return (lane & 3) != 0 || ((lane & 4) && lane != 4) ? -1 : lane & 4 ? 2 : (lane >> 4) * 3 + (lane >> 3 & 1);
 }
 
-// The block's sum of v[q], returned to thread q < 5; fixed order.  sh is free again after the
-// block's next barrier.
+// The block's sum of v[q], returned to thread q < 5; fixed order; only the first `warps` warps hold other
+// numbers than 0.  sh is free again after the block's next barrier.
 template <int NT>
-__device__ __forceinline__ double block_sum5(const double* v, double* sh) {
+__device__ __forceinline__ double block_sum5(const double* v, double* sh, int warps = NT / 32) {
   const double c = warp_sum5(v);
   const int slot = warp_slot();
   if (slot >= 0) sh[(threadIdx.x >> 5) * 5 + slot] = c;
   __syncthreads();
   double t = 0.0;
   if (threadIdx.x < 5)
-#pragma unroll
-    for (int i = 0; i < NT / 32; ++i) t += sh[i * 5 + threadIdx.x];
+#pragma unroll 8
+    for (int i = 0; i < warps; ++i) t += sh[i * 5 + threadIdx.x];
   return t;
 }
 
@@ -568,7 +569,8 @@ __global__ void cyl_final_kernel(const CylCand* __restrict__ cands, const double
   for (long i = threadIdx.x; i < c.nitems; i += CYL_THREADS)
 #pragma unroll
     for (int q = 0; q < 5; ++q) acc[q] += partial[5 * (c.item0 + i) + q];
-  const double t = block_sum5<CYL_THREADS>(acc, sh);
+  // (a small region's sum takes no longer for the block's other warps)
+  const double t = block_sum5<CYL_THREADS>(acc, sh, (int)min((c.nitems + 31) / 32, (long)CYL_THREADS / 32));
   if (threadIdx.x < 5) out[5 * blockIdx.x + threadIdx.x] = t;
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double e = 0.0;

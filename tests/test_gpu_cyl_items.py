@@ -36,3 +36,21 @@ def test_items_of_regions(ctx, reps):
         c1, g1 = one.eval([models[i]])
         assert c1[0] == c32[i] and np.array_equal(g1[0], g32[i])
         at += r[2] * r[3]
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32c"])
+def test_rows_of_regions_of_unequal_height(ctx, precision):
+    """Heights around the rows of a warp (4) and of a block (32) beside a tall region, whose batch launches
+    more rows than the others have: each candidate equals the same candidate alone bit by bit."""
+    rois = [[3, 5, h, 40] for h in (1, 3, 4, 5, 31, 32, 33)] + [[0, 2, 399, 33]]
+    g = hg.QGrid.create(ctx, 516, 420, -2.0, 0.0, 2.0, 3.0, np.deg2rad(0.2), 50.7)
+    rowfc = model.propagation_coeffs(ctx, g, [(4.88e-6, 7.37e-8, 0.0, -1)], 50.7, np.deg2rad(0.2), 0, per_row=True)
+    abc, _ = model.lattice_vectors("hex")
+    models = [fitting.model_block(5 + 0.1 * i, 10 - 0.2 * i, 20 + 0.3 * i, 0.03 * i, 0.05, 11, (20, 20, 1), DN2, (0, 0, 0), 1.0)
+              for i in range(len(rois))]
+    rng = np.random.default_rng(4)
+    counts = [rng.uniform(1, 2, r[2] * r[3]) for r in rois]
+    c, gr = fitting.CylinderBatch(ctx, g, rowfc, abc, rois, np.concatenate(counts), None, 1.0, precision).eval(models)
+    for i, r in enumerate(rois):
+        c1, g1 = fitting.CylinderBatch(ctx, g, rowfc, abc, [r], counts[i], None, 1.0, precision).eval([models[i]])
+        assert c1[0] == c[i] and np.array_equal(g1[0], gr[i])

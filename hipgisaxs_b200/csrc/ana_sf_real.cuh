@@ -63,9 +63,10 @@ __device__ __forceinline__ cx<double> expi_real<double>(double ph) {
 template <>
 __device__ __forceinline__ cx<float> expi_real<float>(double ph) { return expi_turns_real<float>(ph * INV_2PI_R); }
 
-// a / b.  FP64: b's reciprocal by two Newton steps from the FP32 approximation (23 bits) and the quotient
-// corrected by its remainder, without the branches of the IEEE division; rounded as it is but for rare ties, for
-// 1e-37 < |b| < 1e37 (sines and phases here).
+// a / b without the branches of the IEEE division, for 1e-37 < |b| < 1e37 (sines and phases here): b's
+// reciprocal from the approximate one (FP64: two Newton steps), the quotient corrected by its remainder; rounded
+// as the IEEE division is but for rare ties.  CORRECT = false: without the correction, within two ulp.
+template <bool CORRECT = true>
 __device__ __forceinline__ double quotient(double a, double b) {
   float y0;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"((float)b));
@@ -73,9 +74,19 @@ __device__ __forceinline__ double quotient(double a, double b) {
   y = fma(y, fma(-b, y, 1.0), y);
   y = fma(y, fma(-b, y, 1.0), y);
   const double q = a * y;
-  return fma(fma(-b, q, a), y, q);
+  return CORRECT ? fma(fma(-b, q, a), y, q) : q;
 }
-__device__ __forceinline__ float quotient(float a, float b) { return __fdividef(a, b); }
+template <bool CORRECT = true>
+__device__ __forceinline__ float quotient(float a, float b) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+  const float q = a * y;
+  return CORRECT ? fmaf(fmaf(-b, q, a), y, q) : q;
+}
+// The same of a lattice factor: corrected in FP32C, whose sines are as good; in FP64 the rounding of the
+// angles, some 1e-14 of the factor, leaves nothing to correct (7.0e-15 norm-wise either way).
+__device__ __forceinline__ double lattice_quotient(double a, double b) { return quotient<false>(a, b); }
+__device__ __forceinline__ float lattice_quotient(float a, float b) { return quotient(a, b); }
 
 // sin(x) / x (hig::sinc for a real x) given sin x
 __device__ __forceinline__ double sinc_real(double x, double sinx) {

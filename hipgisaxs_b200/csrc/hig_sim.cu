@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(128, 4) grain_dwba_real_kernel(FusedArgs a) {
         const Ratio<T> ra = dirichlet_real<T>(fma(qx, G.a[0], qy * G.a[1]), G.rep[0]);
         // (the phase of a b repetition that is not whole is common to the blocks)
         const Ratio<T> rb = dirichlet_b_real<T>(fma(qx, G.b[0], fma(qy, G.b[1], G.b0)), G.rep[1]);
-        ab = quotient(ra.num * rb.num, ra.den * rb.den);
+        ab = lattice_quotient(ra.num * rb.num, ra.den * rb.den);
         cx<T> v[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) v[k] = f[k];
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(128, 4) grain_dwba_real_kernel(FusedArgs a) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const Ratio<T> rc = dirichlet_real<T>(fma(qz[k], G.c[2], tc), G.rep[2]);
-            v[k] = quotient(rc.num, rc.den) * v[k];
+            v[k] = quotient<false>(rc.num, rc.den) * v[k];  // (ab's correction is the one all blocks share)
           }
         }
         if (G.d[2] != 0.0)  // the rest of the centre's phase is common
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(128, 4) grain_dwba_real_kernel(FusedArgs a) {
           const Ratio<T> ra = dirichlet_real<T>(fma(qx, G.a[0], fma(qy, G.a[1], q * G.a[2])), G.rep[0]);
           const Ratio<T> rb = dirichlet_b_real<T>(ub, G.rep[1]);
           const Ratio<T> rc = dirichlet_real<T>(fma(qx, G.c[0], fma(qy, G.c[1], q * G.c[2])), G.rep[2]);
-          cx<T> v = (quotient(ra.num, ra.den) * quotient(rb.num, rb.den) * quotient(rc.num, rc.den)) * fk;
+          cx<T> v = (lattice_quotient(ra.num, ra.den) * lattice_quotient(rb.num, rb.den) * lattice_quotient(rc.num, rc.den)) * fk;
           if (G.rep[1] != round_fp64(G.rep[1])) v = v * b_phase_real<T>(ub, G.rep[1]);
           if (G.d[0] != 0.0 || G.d[1] != 0.0 || G.d[2] != 0.0)
             v = v * expi_turns_real<T>(fma(qx, G.d[0], fma(qy, G.d[1], q * G.d[2])));

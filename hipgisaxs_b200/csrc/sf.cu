@@ -74,11 +74,11 @@ __global__ void __launch_bounds__(128) sf_lattice_real_kernel(SfRealArgs a) {
       const double ub = fma(qx, a.b[0], fma(qy, a.b[1], fma(qz, a.b[2], a.b0)));
       const Ratio<T> ra = dirichlet_real<T>(fma(qx, a.a[0], fma(qy, a.a[1], qz * a.a[2])), a.rep[0]);
       const Ratio<T> rb = dirichlet_b_real<T>(ub, a.rep[1]);
-      ab = quotient(ra.num, ra.den) * quotient(rb.num, rb.den);
+      ab = lattice_quotient(ra.num, ra.den) * lattice_quotient(rb.num, rb.den);
       if (!whole) bp = b_phase_real<T>(ub, a.rep[1]);
     }
     const Ratio<T> rc = dirichlet_real<T>(fma(qx, a.c[0], fma(qy, a.c[1], qz * a.c[2])), a.rep[2]);
-    cx<T> v = (ab * quotient(rc.num, rc.den)) * bp;
+    cx<T> v = (ab * lattice_quotient(rc.num, rc.den)) * bp;
     if (moved) v = v * expi_turns_real<T>(fma(qx, a.d[0], fma(qy, a.d[1], qz * a.d[2])));
     OUT* out = reinterpret_cast<OUT*>(a.out) + k * a.n + i;
     out->x = v.x;

@@ -1,5 +1,6 @@
 // Fixed-point digits for tcgen05.mma kind::i8, shared by the triangle form factor (ff_tri_mma.cu) and
-// its adjoint (mesh_adjoint_mma.cu): numbers as three signed 8-bit digits, value = d0 2^16 + d1 2^8 + d2.
+// its adjoint (mesh_adjoint_mma.cu): phasors as three signed 8-bit digits, value = d0 2^16 + d1 2^8 + d2, the
+// other factor as four.
 #pragma once
 
 #include "ff_tri.cuh"
@@ -9,20 +10,35 @@ namespace hgx {
 constexpr int MMA_K = 32;                     // triangles per product
 constexpr float A_SCALE = 4161344.0f;         // |c| <= 1 -> below 2^22 - 0x8080, so the sum below stays under 2^23
 constexpr float A_MAGIC = 12615808.0f;        // 2^23 + 2^22 + 0x8080: low mantissa bits = a + 2^22 + 0x8080
-constexpr double B_SCALE = 8355000.0;         // the largest |n~| of a tile (three signed digits reach 0x7f7f7f)
-constexpr double V_UNIT = 16777216.0 / (4161344.0 * 8355000.0);  // one unit of the combined sum (2^24 products)
+constexpr double B_SCALE = 8355000.0 * 256.0; // the largest of the other factor (four signed digits reach 0x7f7f7f7f)
+// One unit (2^16 products) of the combined sum.  The sums are taken in units of 2^36 of these and the scales
+// times 2^36 (about half the largest factor), so that neither leaves the range of FP32 where the factors do not.
+constexpr float S36 = 1.0f / 68719476736.0f;
+constexpr double V_UNIT = 65536.0 / (4161344.0 * B_SCALE) * 68719476736.0;
 
 constexpr int A_COLS = 6 * MMA_K / 4;          // TMEM columns of a warpgroup's digits (2 x 3 planes of 8)
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) { return __byte_perm(a, b, sel); }
 
-// The digit planes of four integers b_i = w_i - 0x808080, |b_i| <= 0x7f7f7f, one byte each.
-__device__ __forceinline__ void signed_digits(const uint32_t (&w)[4], uint32_t (&dig)[3]) {
+// The digit planes of four integers b_i = w_i - 0x80808080, |b_i| <= 0x7f7f7f7f, one byte each.
+__device__ __forceinline__ void signed_digits(const uint32_t (&w)[4], uint32_t (&dig)[4]) {
   const uint32_t p01 = prmt(w[0], w[1], 0x5140), p23 = prmt(w[2], w[3], 0x5140);
-  const uint32_t h01 = prmt(w[0], w[1], 0x0062), h23 = prmt(w[2], w[3], 0x0062);
-  dig[0] = prmt(h01, h23, 0x5410) ^ 0x80808080u;
-  dig[1] = prmt(p01, p23, 0x7632) ^ 0x80808080u;
-  dig[2] = prmt(p01, p23, 0x5410) ^ 0x80808080u;
+  const uint32_t h01 = prmt(w[0], w[1], 0x7362), h23 = prmt(w[2], w[3], 0x7362);
+  dig[0] = prmt(h01, h23, 0x7632) ^ 0x80808080u;
+  dig[1] = prmt(h01, h23, 0x5410) ^ 0x80808080u;
+  dig[2] = prmt(p01, p23, 0x7632) ^ 0x80808080u;
+  dig[3] = prmt(p01, p23, 0x5410) ^ 0x80808080u;
+}
+
+// The offset of 64 of the phasors' top digits adds 2^22 sum(b) to a column's sum: in units of 2^32, and the rest
+// in the combined sum's.
+__device__ __forceinline__ uint32_t offset_units(long long sum) { return (uint32_t)(sum >> 10); }
+__device__ __forceinline__ float offset_rest(long long sum) { return (float)((int)(sum & 1023) << 6) * S36; }
+// A column's combined sum less that offset, from its four accumulators s_i (weights 2^24, 2^16, 2^8, 1 units).
+__device__ __forceinline__ float combined_sum(uint32_t s0, uint32_t s1, uint32_t s2, uint32_t s3, uint32_t units,
+                                              float rest) {
+  const float lo = fmaf((float)(int)s2, 256.f * S36, fmaf((float)(int)s3, S36, -rest));
+  return fmaf((float)(int)(s0 * 256u + s1 - units), 65536.f * S36, lo);
 }
 
 // The digits of the phasors e^{i q.d} of this thread's q with 16 offsets d (or of its offset with

@@ -7,17 +7,20 @@
 // so the tile needs sum_t c_t b_tj and sum_t s_t b_tj with the six real columns
 // b = (n~x, n~y, n~z) x (Re Z, Im Z) per block pair (qz, -qz) or per complex block.
 //
-// Both factors become 24-bit fixed-point integers cut into three signed 8-bit digits
-// (value = d0 2^16 + d1 2^8 + d2): |c|, |s| <= 1 with step 1 / 4161344 (about 2^-22), the row
-// factors relative to the tile's largest |n~| (step 2^-23).  The products of digits with
-// i + j <= 2 accumulate exactly in 32-bit integers (tcgen05.mma kind::i8, A = the phasors in
-// TMEM, B = the row factors in shared memory, accumulators in TMEM):
-//   A0 x [B0 B1 B2], A1 x [B0 B1], A2 x [B0], the slices offset so that equal i + j add up.
-// What is left out is below 2^-29 of a term, and the accumulation itself has no rounding error,
-// so the SFU's own error (about 2^-22) stays the largest, as in the FP32 kernel.
+// Both factors become fixed-point integers cut into signed 8-bit digits: |c|, |s| <= 1 with step
+// 1 / 4161344 (about 2^-22) into three, the row factors relative to the tile's largest |n~| (step
+// 2^-31, so that those of triangles of 2^-7 of the largest still have their 24 bits) into four.  The
+// products of digits with i + j <= 3 accumulate exactly in 32-bit integers (tcgen05.mma kind::i8, A =
+// the phasors in TMEM, B = the row factors in shared memory, accumulators in TMEM):
+//   A0 x [B0 B1 B2 B3], A1 x [B0 B1 B2], A2 x [B0 B1], the slices offset so that equal i + j add up.
+// What is left out is below 2^-29 of a term, and the accumulation itself has no rounding error.
+// Norm-wise error over the FP32 row kernel's: 0.6 to 0.7 on closed meshes of even and of uneven
+// triangles, 0.3 to 0.5 on complex blocks (with three digits, step 2^-23: 0.7 on even ones, up to 3 on uneven
+// ones, and 5 to 11 on complex blocks), 1.2 where pairs of opposite faces a thousandth of a nm apart cancel
+// to 1e-4, where the phasors' step shows.
 //
 // A CTA (one per SM) owns 128 columns of one detector row, the 128 TMEM lanes, and a range of
-// tiles.  Five warpgroups (six on complex blocks) take its chunks of 32 triangles in turn: each
+// tiles.  Five warpgroups take its chunks of 32 triangles in turn: each
 // thread makes its pixel's digits and stores them to its warpgroup's part of TMEM; two more warps
 // issue the products with cos and with sin.  On real blocks the accumulators alternate between
 // two column ranges, so that a tile's sums are read back, scaled, rotated by the tile's FP64
@@ -26,10 +29,10 @@
 //
 // What bounds it: the digits.  Per (pixel, triangle) two SFU operations and about 14 issued
 // instructions (PRMT 3.6, FFMA2 1.5, LOP3 1.3, FMUL 1.2): SFU 76%, issue 66%; the products take
-// 100 of the 680 cycles of a chunk.  2048 x 2048 x 50,000: 127 ms with 20 digit warps of 80
-// registers (24 of 72: 129; 16 of 96: 147; three warpgroups of 168 registers, each with its own
-// pixels: 148), against 190 ms for the FP32 row kernel, whose 16 FFMA per (pixel, triangle) of
-// accumulation these products replace.  Taking a quarter of the sines off the SFU by polynomials on the
+// 150 of the 690 cycles of a chunk.  2048 x 2048 x 50,000: 129 ms with 20 digit warps of 80
+// registers (with three digits of the row factors 126, and then 24 warps of 72: 129, 16 of 96: 147, three
+// warpgroups of 168 registers, each with its own pixels: 148), against 190 ms for the FP32 row kernel, whose 16
+// FFMA per (pixel, triangle) of accumulation these products replace.  Taking a quarter of the sines off the SFU by polynomials on the
 // FMA pipe left the time unchanged.
 //
 // The row factors of a slab of rows are made once per (row, triangle) by ff_row_factor_kernel,
@@ -55,16 +58,16 @@ template <int U>
 struct MmaShape {
   static constexpr int NP = U == 4 ? 32 : 16;           // columns per digit slice (6 U, padded)
   static constexpr int SBO = 128;
-  static constexpr int LBO = 3 * NP / 8 * 128;
+  static constexpr int LBO = 4 * NP / 8 * 128;
   static constexpr int CHUNK_BYTES = 2 * LBO;           // row factors of 32 triangles
   static constexpr int TILE_B_BYTES = MMA_CHUNKS * CHUNK_BYTES;
   static constexpr int XY_BYTES = MMA_XY * 4;
-  static constexpr int REC = U == 4 ? 32 : (U == 2 ? 16 : 8);  // words per (row, tile) record
+  static constexpr int REC = (13 * U + 3) / 4 * 4;      // words per (row, tile) record
   static constexpr int STAGE = TILE_B_BYTES + XY_BYTES + REC * 4;  // one tile in shared memory
-  static constexpr int NST = U == 4 ? 3 : 4;            // tiles in shared memory
-  static constexpr int D_COLS = 3 * NP;                 // accumulator columns of cos, then of sin
+  static constexpr int NST = U == 4 ? 2 : 4;            // tiles in shared memory
+  static constexpr int D_COLS = 4 * NP;                 // accumulator columns of cos, then of sin
   static constexpr int DBUF = U == 4 ? 1 : 2;           // accumulator ranges
-  static constexpr int SUB = U == 4 ? 6 : 5;            // warpgroups making digits
+  static constexpr int SUB = 5;                         // warpgroups making digits
   static constexpr int THREADS = SUB * 128 + 64;        // and two warps that issue the products
   static constexpr int NACC = U == 1 ? 2 : 8;           // sums per pixel
   static constexpr int SUM_BYTES = SUB * NACC * 128 * 8;  // FP64 sums of each warpgroup
@@ -79,13 +82,13 @@ struct FactorArgs {
   const double2* rowqz;    // nrow x NK
   int ntiles, row0, nrows; // slab rows
   unsigned char* b;        // [slab row][tile] TILE_B_BYTES
-  uint32_t* rec;           // [slab row][tile] REC words: 6 U column sums / 4, U scales (float)
+  uint32_t* rec;           // [slab row][tile] REC words: 6 U offsets, U scales, 6 U offsets' rests
 };
 
 constexpr int FACTOR_THREADS = TILE / 4;
 
 // One CTA per tile and group of rows, four triangles per thread (one 32-bit word of each digit
-// plane).  The digits are biased by 0x80 (b2, b1, b0 of b + 0x808080) and flipped back to signed
+// plane).  The digits are biased by 0x80 (the bytes of b + 0x80808080) and flipped back to signed
 // bytes; the tile's image is put together in shared memory and written out in 16-byte words.
 // About 200 instructions per (row, triangle), 1% of the products' time at 2048 columns.
 template <int U, bool PAIRED>
@@ -93,7 +96,7 @@ __global__ void __launch_bounds__(FACTOR_THREADS) ff_row_factor_kernel(FactorArg
   using S = MmaShape<U>;
   constexpr int NK = PAIRED ? 4 : U;
   extern __shared__ __align__(16) unsigned char s_img[];
-  __shared__ int s_sum[FACTOR_THREADS / 32][6 * U];
+  __shared__ long long s_sum[FACTOR_THREADS / 32][6 * U];
   const int tile = blockIdx.x, t = threadIdx.x;
   const double4 anc = a.anchors[tile];
   const float4 info = a.info[tile];
@@ -149,22 +152,24 @@ __global__ void __launch_bounds__(FACTOR_THREADS) ff_row_factor_kernel(FactorArg
 #pragma unroll
       for (int j = 0; j < 6; ++j) {
         uint32_t w[4];
-        int sum = 0;
+        int hi = 0, lo = 0;  // of the sum of b, so that a warp's fits
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int b = __float2int_rn(n[i][j % 3] * (j < 3 ? re[i] : im[i]));
-          sum += b;
-          w[i] = (uint32_t)(b + 0x808080);
+          hi += b >> 8;
+          lo += b & 255;
+          w[i] = (uint32_t)b + 0x80808080u;
         }
-        uint32_t dig[3];
+        uint32_t dig[4];
         signed_digits(w, dig);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
+        for (int d = 0; d < 4; ++d) {
           const int col = d * S::NP + 6 * u + j;
           *reinterpret_cast<uint32_t*>(s_img + base + (col >> 3) * S::SBO + (col & 7) * 16) = dig[d];
         }
-        const int ws = __reduce_add_sync(0xffffffffu, sum);  // at most 128 x 2^23
-        if ((t & 31) == 0) s_sum[t >> 5][6 * u + j] = ws;
+        hi = __reduce_add_sync(0xffffffffu, hi);  // at most 128 x 2^23
+        lo = __reduce_add_sync(0xffffffffu, lo);
+        if ((t & 31) == 0) s_sum[t >> 5][6 * u + j] = (long long)hi * 256 + lo;
       }
       if (t == 0)
         a.rec[cell * S::REC + 6 * U + u] = __float_as_uint((float)((double)info.x * V_UNIT * top));
@@ -173,11 +178,10 @@ __global__ void __launch_bounds__(FACTOR_THREADS) ff_row_factor_kernel(FactorArg
     uint4* dst = reinterpret_cast<uint4*>(a.b + cell * S::TILE_B_BYTES);
     for (int i = t; i < S::TILE_B_BYTES / 16; i += FACTOR_THREADS) dst[i] = reinterpret_cast<const uint4*>(s_img)[i];
     if (t < 6 * U) {
-      // the phasors' top digit keeps an offset of 64 (2^22 in their units): 2^22 x (sum of b) comes
-      // off again in units of 2^24
-      long long v = 2;
+      long long v = 0;
       for (int w = 0; w < FACTOR_THREADS / 32; ++w) v += s_sum[w][t];
-      a.rec[cell * S::REC + t] = (uint32_t)(v >> 2);
+      a.rec[cell * S::REC + t] = offset_units(v);
+      a.rec[cell * S::REC + 7 * U + t] = __float_as_uint(offset_rest(v));
     }
     __syncthreads();
   }
@@ -238,14 +242,14 @@ __device__ __forceinline__ void add_tile_sums(const MmaArgs& a, uint32_t d_tm, i
     float f[2][6];  // sums with cos, with sin: (n~x, n~y, n~z) Re Z, then Im Z
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      uint32_t d[24];
+      uint32_t d[32];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) tmem_ld8(d_tm + k * S::D_COLS + i * S::NP + 6 * u, d + 8 * i);
-      tmem_wait_ld<24>(d);
+      for (int i = 0; i < 4; ++i) tmem_ld8(d_tm + k * S::D_COLS + i * S::NP + 6 * u, d + 8 * i);
+      tmem_wait_ld<32>(d);
 #pragma unroll
       for (int j = 0; j < 6; ++j)
-        // (s0 2^16 + s1 2^8 + s2) / 2^8 less the top digit's offset
-        f[k][j] = (float)((int)(d[j] * 256u + d[8 + j] - rec[6 * u + j]) + (((int)d[16 + j] + 128) >> 8));
+        f[k][j] = combined_sum(d[j], d[8 + j], d[16 + j], d[24 + j], rec[6 * u + j],
+                               __uint_as_float(rec[7 * U + 6 * u + j]));
     }
     const float *fc = f[0], *fs = f[1];
     const double2 q = a.rowqz[(long)row * NK + (PAIRED ? 2 * u : u)];
@@ -539,9 +543,9 @@ __global__ void __launch_bounds__(MmaShape<U>::THREADS, 1) ff_tri_mma_kernel(Mma
         __syncwarp();
         const uint32_t av = tm_a + k * A_COLS + 24 * t;
         if (elect_one()) {
-          mma_s8_ts(dc, av, bd, idesc_s8(3 * S::NP), ch > 0);
-          mma_s8_ts(dc + S::NP, av + 8, bd, idesc_s8(2 * S::NP), 1);
-          mma_s8_ts(dc + 2 * S::NP, av + 16, bd, idesc_s8(S::NP), 1);
+          mma_s8_ts(dc, av, bd, idesc_s8(4 * S::NP), ch > 0);
+          mma_s8_ts(dc + S::NP, av + 8, bd, idesc_s8(3 * S::NP), 1);
+          mma_s8_ts(dc + 2 * S::NP, av + 16, bd, idesc_s8(2 * S::NP), 1);
           mma_commit(&s_used[k]);
         }
         __syncwarp();

@@ -56,20 +56,6 @@ constexpr int BWM_SUMS = BWM_SUB * 6 * 128 * 8;
 constexpr int BWM_NREC = 4;                   // items whose records are held
 constexpr int BWM_SMEM = BWM_NST * BWM_STAGE + BWM_NREC * BWM_REC * 4 + BWM_SUMS;
 constexpr int BWM_D = BWM_ND * BWM_NP;        // accumulator columns, two ranges
-// The combined sums are taken in units of 2^36 and the scales times 2^36 (about half the column's
-// largest modulus), so that neither leaves the range of FP32 where the moduli do not.
-constexpr float BWM_S36 = 1.0f / 68719476736.0f;
-constexpr double BWM_UNIT = V_UNIT / 65536.0 * 68719476736.0;
-
-// The digit planes of four integers b_i = w_i - 0x80808080, |b_i| <= 0x7f7f7f7f.
-__device__ __forceinline__ void signed_digits4(const uint32_t (&w)[4], uint32_t (&dig)[4]) {
-  const uint32_t p01 = prmt(w[0], w[1], 0x5140), p23 = prmt(w[2], w[3], 0x5140);
-  const uint32_t h01 = prmt(w[0], w[1], 0x7362), h23 = prmt(w[2], w[3], 0x7362);
-  dig[0] = prmt(h01, h23, 0x7632) ^ 0x80808080u;
-  dig[1] = prmt(h01, h23, 0x5410) ^ 0x80808080u;
-  dig[2] = prmt(p01, p23, 0x7632) ^ 0x80808080u;
-  dig[3] = prmt(p01, p23, 0x5410) ^ 0x80808080u;
-}
 
 // Column j of a pair's 12: weight and which number of (P, M).
 //   0 ReP qx, 1 ImM qx, 2 ReP qy, 3 ImM qy, 4 ImP, 5 ReM, 6 ImP qx^2, 7 ReM, 8 ImP qx qy, 9 ReM, 10 ImP qy^2, 11 ReM
@@ -168,7 +154,7 @@ __global__ void __launch_bounds__(256) bwm_seed_kernel(BwmArgs a, int row0) {
     if (j < 12) {
       // two factors where one would leave FP32's range
       const float top = a.colmax[(size_t)item * 24 + 12 * pr + j], up = top < 0x1p-60f ? 0x1p64f : 1.f;
-      const float sc = (float)(B_SCALE * 256.0 / ((double)top * (double)up));
+      const float sc = (float)(B_SCALE / ((double)top * (double)up));
       int hi = 0, lo = 0;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -177,7 +163,7 @@ __global__ void __launch_bounds__(256) bwm_seed_kernel(BwmArgs a, int row0) {
         lo += b & 255;
         x[i] = (uint32_t)b + 0x80808080u;
       }
-      signed_digits4(x, dig);
+      signed_digits(x, dig);
       hi = __reduce_add_sync(0xffffffffu, hi);
       lo = __reduce_add_sync(0xffffffffu, lo);
       if ((t & 31) == 0) s_sum[threadIdx.x >> 5][j] = (long long)hi * 256 + lo;
@@ -197,14 +183,13 @@ __global__ void __launch_bounds__(256) bwm_seed_kernel(BwmArgs a, int row0) {
     dst[i] = *reinterpret_cast<const uint4*>(s_img + i / (4 * HALF) * BWM_IMG_CHUNK + (i / HALF & 3) * BWM_IMG_LBO +
                                              i % HALF * 16);
   if (threadIdx.x < 24) {
-    // the top phasor digits' offset of 64 adds 2^22 sum(b): in units of 2^32, and the rest of 2^16
     const int c = threadIdx.x, w0 = c / 12 * 2, j = c % 12;
     const long long off = s_sum[w0][j] + s_sum[w0 + 1][j] + s_sum[w0 + 4][j] + s_sum[w0 + 5][j];
     const float top = a.colmax[(size_t)item * 24 + c];
     uint32_t* rec = a.rec + cell * BWM_REC + c;
-    rec[0] = (uint32_t)(off >> 10);
-    rec[24] = __float_as_uint(top == INFINITY ? NAN : (float)((double)top * BWM_UNIT));
-    rec[48] = __float_as_uint((float)((int)(off & 1023) << 6) * BWM_S36);
+    rec[0] = offset_units(off);
+    rec[24] = __float_as_uint(top == INFINITY ? NAN : (float)((double)top * V_UNIT));
+    rec[48] = __float_as_uint(offset_rest(off));
   }
 }
 
@@ -225,9 +210,7 @@ __device__ __forceinline__ void bwm_add(uint32_t d_tm, const uint32_t* rec, doub
       for (int j = 0; j < 8; ++j) {
         const int c = 12 * pr + 8 * h + j;
         if (8 * h + j < 12) {
-          const float lo = fmaf((float)(int)d[16 + j], 256.f * BWM_S36,
-                                fmaf((float)(int)d[24 + j], BWM_S36, -__uint_as_float(rec[48 + c])));
-          f[8 * h + j] = fmaf((float)(int)(d[j] * 256u + d[8 + j] - rec[c]), 65536.f * BWM_S36, lo) *
+          f[8 * h + j] = combined_sum(d[j], d[8 + j], d[16 + j], d[24 + j], rec[c], __uint_as_float(rec[48 + c])) *
                          __uint_as_float(rec[24 + c]);
         }
       }

@@ -91,3 +91,30 @@ def test_both_sides_of_the_kernel_choice(ctx, po, ncol, nrow, ntri):
     qx, qy, qz = detector(po, ncol, nrow, "real")
     g = hg.QGrid.from_arrays(ctx, qx, qy, qz, ncol)
     assert po.rel_err(hg.ff_triangles(ctx, g, sd, None, "f32c"), po.ff_approx_triangle(sd, qx, qy, qz)) < TOL32
+
+
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("spread", [1.0, 3.0])
+def test_triangles_of_uneven_size(ctx, po, kind, spread):
+    """Areas over orders of magnitude (log-normal): what a term is off is that of the SFU's sine and cosine
+    (2^-21.4) and of the phasors' step (2^-23), 5e-7 of the term, and adds up at random: 1e-6 norm-wise, the error
+    of the sums of even triangles, not that of the tile's largest triangle times their number."""
+    sd = cloud(np.random.default_rng(3), 600)
+    sd[:, 0] = np.exp(spread * np.random.default_rng(4).normal(size=600))
+    qx, qy, qz = detector(po, 256, 40, kind)
+    g = hg.QGrid.from_arrays(ctx, qx, qy, qz, 256)
+    ref = po.ff_approx_triangle(sd, qx, qy, qz)
+    f = hg.ff_triangles(ctx, g, sd, None, "f32c")
+    ok = np.isfinite(ref)
+    assert po.rel_err(f[ok], ref[ok]) < 1e-6
+
+
+@pytest.mark.parametrize("unit", [1e-33, 1e30])
+def test_units_of_the_areas(ctx, po, unit):
+    sd = cloud(np.random.default_rng(3), 600)
+    sd[:, 0] *= unit
+    qx, qy, qz = detector(po, 256, 8, "real")
+    g = hg.QGrid.from_arrays(ctx, qx, qy, qz, 256)
+    ref = po.ff_approx_triangle(sd, qx, qy, qz)
+    ok = np.isfinite(ref)
+    assert po.rel_err(hg.ff_triangles(ctx, g, sd, None, "f32c")[ok], ref[ok]) < TOL32

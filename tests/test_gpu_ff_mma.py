@@ -118,3 +118,25 @@ def test_units_of_the_areas(ctx, po, unit):
     ref = po.ff_approx_triangle(sd, qx, qy, qz)
     ok = np.isfinite(ref)
     assert po.rel_err(hg.ff_triangles(ctx, g, sd, None, "f32c")[ok], ref[ok]) < TOL32
+
+
+@pytest.mark.parametrize("along", ["qy", "qx"])
+@pytest.mark.parametrize("width,ncol", [(0.02, 130), (0.1, 130), (0.01, 1)])
+def test_zoomed_grids_around_zero(ctx, po, along, width, ncol):
+    """Point by point next to q = 0, where F = S / q^2 and S cancels: a term is off by 5e-7 of |q| |n|, so F by
+    5e-7 |q| (surface) / (|q|^2 volume), 3e-6 / (|q| D) for a ball of diameter D; 5e-6 (1 + 1 / (|q| D)) allowed."""
+    V, F = meshes.star_mesh(15.0, 64, 33)
+    sd = meshes.shape_def_from_mesh(V, F)
+    nrow = 160
+    u = np.tile(np.linspace(-width, 1.01 * width, ncol) if ncol > 1 else 1e-4, nrow)
+    v = np.full(ncol * nrow, 1e-5)
+    qx, qy = (v, u) if along == "qy" else (u, v)
+    z = np.repeat(np.linspace(1e-4, width, nrow), ncol).astype(complex)
+    a, b = z + 1e-4, z - 5e-5
+    qz = np.concatenate([a, -b, b, -a])
+    g = hg.QGrid.from_arrays(ctx, qx, qy, qz, ncol)
+    assert g.mode == 1
+    qd = 30.0 * np.sqrt(np.tile(qx ** 2 + qy ** 2, 4) + qz.real ** 2)
+    ref = hg.ff_triangles(ctx, g, sd, None, "f64")
+    e = np.abs(hg.ff_triangles(ctx, g, sd, None, "f32c") - ref) / np.abs(ref)
+    assert np.all(e[qd < 2] < 5e-6 * (1 + 1 / qd[qd < 2]))

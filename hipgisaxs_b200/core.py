@@ -186,8 +186,9 @@ TUNE_CANDIDATES = (4, 2, 1, -2, -4, -8)
 
 
 def ff_tune(ctx: Context, grid: QGrid, shape_def, rot=None, out_type="c64", reps=2):
-    """Autotune the FP32C kernel's launch shape on `grid` (hgx_ff_tune); later automatic
-    calls on this grid use the choice.  Returns (pixels_per_thread, ms, {candidate: ms})."""
+    """Autotune the FP32C row kernels on `grid` (hgx_ff_tune): the FP32 kernel's launch shapes and
+    the tensor-core kernel; later automatic calls on this grid use the choice.  Returns
+    (pixels_per_thread, ms, {shape: ms}); pixels_per_thread is 0 when no shape is the fastest."""
     psd, ksd = _in(shape_def, np.float64)
     ntri = int((ksd.numel() if _is_tensor(ksd) else ksd.size) // 8)
     r = _rot_arg(rot)

@@ -1169,6 +1169,9 @@ static bool rows_mma_pays(hgx_ctx c, hgx_qgrid g, int ntri) {
   return !(fp32 < 0.9 * mma);
 }
 
+constexpr int WANT_MMA = 1 << 20;  // want_p of the autotuner's tensor-core candidate (refused from callers)
+static const char PIXELS_REFUSED[] = "hgx_ff_triangles: pixels per thread must be 1, 2 or 4 (scalar) or -2, -4, -8 (packed)";
+
 int ff_triangles_device(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, const double* rot9,
                         int precision, void* out, int ff_type, int want_p) {
   cudaStream_t st = c->stream;
@@ -1186,19 +1189,19 @@ int ff_triangles_device(hgx_ctx c, hgx_qgrid g, const double* sd, int ntri, cons
     HGX_CUDA(cudaGetLastError());
     return HGX_OK;
   }
-  if (want_p == 0 && g->tuned_p == 0 && g->mode != 0 && rows_mma_pays(c, g, ntri)) {
+  if (g->mode != 0 && (want_p == WANT_MMA || (want_p == 0 && g->tuned_p == 0 && rows_mma_pays(c, g, ntri)))) {
     if (row_shape(g->nrow, g->ncol, c->sm_count, 4).grid.y > 65535u)
       return fail(HGX_ERR_INVALID_ARG, "hgx_ff_triangles: too many detector rows for one launch");
     TilePrep t;
     HGX_TRY(prepare_tiles(c, sd, ntri, R, false, &t));
     const int s = ff_rows_mma(c, g, MmaTiles{t.tiles, t.anchors, t.xy, t.info, c->tiles.ntiles, ntri}, R, out, ff_type);
-    if (s != HGX_ERR_NO_MEMORY) return s;  // without room for the row factors: the row kernels below
+    // without room for the row factors: the row kernels below
+    if (s != HGX_ERR_NO_MEMORY || want_p == WANT_MMA) return s;
   }
   if (want_p == 0) want_p = g->tuned_p;  // the autotuner's choice for this grid, if any
   if (want_p != 0 && want_p != 1 && want_p != 2 && want_p != 4 && want_p != -2 && want_p != -4 &&
       want_p != -8)
-    return fail(HGX_ERR_INVALID_ARG, "hgx_ff_triangles: pixels per thread must be 1, 2 or 4 (scalar) "
-                                     "or -2, -4, -8 (packed)");
+    return fail(HGX_ERR_INVALID_ARG, PIXELS_REFUSED);
   const int ntiles = (ntri + TILE - 1) / TILE;
   // paired real DWBA blocks, packed FP32x2 kernel on request (want_p = -2, -4, -8 pixels per
   // thread); automatic (0) picks the scalar one.
@@ -1302,6 +1305,7 @@ int hgx_ff_triangles_q_ex(hgx_ctx c, hgx_qgrid g, const double* shape_def, int n
   if (ff_type != HGX_C128 && ff_type != HGX_C64)
     return fail(HGX_ERR_INVALID_ARG, "hgx_ff_triangles_q: unknown output type");
   if (g->ctx != c) return fail(HGX_ERR_INVALID_ARG, "hgx_ff_triangles_q: grid of another context");
+  if (precision == HGX_F32C && pixels == WANT_MMA) return fail(HGX_ERR_INVALID_ARG, PIXELS_REFUSED);
   HGX_CUDA(cudaSetDevice(c->device));
   cudaStream_t st = c->stream;
   const double* sd = nullptr;
@@ -1320,9 +1324,11 @@ int hgx_ff_triangles_q(hgx_ctx c, hgx_qgrid g, const double* shape_def, int ntri
   return hgx_ff_triangles_q_ex(c, g, shape_def, ntri, rot9, precision, ff, ff_type, 0);
 }
 
-// The launch-shape autotuner of the FP32C row kernel.  Candidates, in this order: scalar
+// The autotuner of the FP32C row kernels.  Candidates, in this order: scalar
 // kernel with 4, 2, 1 pixels per thread, then (paired real grids only) the packed FP32x2
-// kernel with 2, 4, 8.  Each is run once untimed and then `reps` times between two CUDA
+// kernel with 2, 4, 8, then the tensor-core kernel (on paired real grids from the second tile of
+// triangles on: with one tile the two kinds are within 15% of each other and of the launches' noise, and
+// the shapes alone are ranked).  When it wins nothing is stored.  Each is run once untimed and then `reps` times between two CUDA
 // events on the context's stream, on the caller's triangles (the cost of every candidate is
 // linear in the triangle count, so a few thousand triangles rank them); the fastest is stored
 // in the grid and used by later calls that ask for the automatic shape.
@@ -1366,11 +1372,14 @@ int hgx_ff_tune(hgx_ctx c, hgx_qgrid g, const double* shape_def, int ntri, const
   HGX_CUDA(cudaEventCreate(&ev.e[0]));
   HGX_CUDA(cudaEventCreate(&ev.e[1]));
   int best = 0;
-  double bms = 0.0;
-  for (int i = 0; i < TUNE_NCAND; ++i) {
-    const int p = TUNE_CANDIDATES[i];
-    if (p < 0 && g->mode != 1) continue;
-    HGX_TRY(ff_triangles_device(c, g, sd, ntri, rot9, HGX_F32C, out.p, ff_type, p));
+  double bms = -1.0;
+  for (int i = 0; i <= TUNE_NCAND; ++i) {
+    const bool mma = i == TUNE_NCAND;
+    const int p = mma ? WANT_MMA : TUNE_CANDIDATES[i];
+    if ((p < 0 && g->mode != 1) || (mma && g->mode == 1 && ntri <= TILE)) continue;
+    const int s = ff_triangles_device(c, g, sd, ntri, rot9, HGX_F32C, out.p, ff_type, p);
+    if (mma && s == HGX_ERR_NO_MEMORY) break;  // later calls would not take it either
+    if (s != HGX_OK) return s;
     HGX_CUDA(cudaEventRecord(ev.e[0], st));
     for (int r = 0; r < reps; ++r)
       HGX_TRY(ff_triangles_device(c, g, sd, ntri, rot9, HGX_F32C, out.p, ff_type, p));
@@ -1379,9 +1388,9 @@ int hgx_ff_tune(hgx_ctx c, hgx_qgrid g, const double* shape_def, int ntri, const
     float ms = 0.f;
     HGX_CUDA(cudaEventElapsedTime(&ms, ev.e[0], ev.e[1]));
     double per = (double)ms / reps;
-    if (times_ms) times_ms[i] = per;
-    if (best == 0 || per < bms) {
-      best = p;
+    if (times_ms && !mma) times_ms[i] = per;
+    if (bms < 0.0 || per < bms) {
+      best = mma ? 0 : p;
       bms = per;
     }
   }

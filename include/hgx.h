@@ -101,21 +101,22 @@ int hgx_ff_triangles_q(hgx_ctx ctx, hgx_qgrid g, const double* shape_def, int nt
                        const double* rot9, int precision, void* ff, int ff_type);
 /* As hgx_ff_triangles_q with an explicit launch shape for the FP32 row kernel:
  * pixels_per_thread 1, 2 or 4 selects the scalar kernel with that many pixels per thread;
- * -2, -4 or -8 the packed FP32x2 kernel (paired real grids only); 0 = automatic (on row grids
- * nearly always the tensor-core kernel, which has one shape and keeps up to 1 GiB of row factors
- * in the context; else the shape hgx_ff_tune stored, or scalar with 4, fewer when the grid is too
- * small to fill the GPU). */
+ * -2, -4 or -8 the packed FP32x2 kernel (paired real grids only); 0 = automatic: the shape that
+ * hgx_ff_tune stored in the grid if any, else on row grids nearly always the tensor-core kernel (which
+ * has one shape and keeps up to 1 GiB of row factors in the context), else scalar with 4, fewer when the
+ * grid is too small to fill the GPU. */
 int hgx_ff_triangles_q_ex(hgx_ctx ctx, hgx_qgrid g, const double* shape_def, int ntri,
                           const double* rot9, int precision, void* ff, int ff_type,
                           int pixels_per_thread);
-/* The launch-shape autotuner of the FP32 row kernel (no reference counterpart; the reference
- * launches one fixed shape).  Times the candidate pixels_per_thread values 4, 2, 1 (scalar)
- * and, on paired real grids, -2, -4, -8 (packed) on these triangles — one untimed launch,
- * then `reps` launches between CUDA events each — and stores the fastest in the grid, where
- * later calls with the automatic shape (hgx_ff_triangles_q, or pixels_per_thread 0) use it
- * instead of the tensor-core kernel, which most grids run faster on untuned.
+/* The autotuner of the FP32C row kernels (no reference counterpart; the reference
+ * launches one fixed shape).  Times the FP32 row kernel with the pixels_per_thread values 4, 2, 1
+ * (scalar) and, on paired real grids, -2, -4, -8 (packed), and the tensor-core kernel (on paired real
+ * grids with more than 512 triangles), on these triangles — one untimed launch,
+ * then `reps` launches between CUDA events each.  When a shape of the FP32 kernel is the fastest it is
+ * stored in the grid, where later calls with the automatic shape (hgx_ff_triangles_q, or
+ * pixels_per_thread 0) use it; when the tensor-core kernel is, nothing is stored and best_ppt = 0.
  * Cost is linear in ntri for every candidate, so a few thousand triangles rank them.
- * best_ppt, best_ms and times_ms (6 means in the order above; 0 for a candidate the grid
+ * best_ppt, best_ms and times_ms (the 6 shapes' means in the order above; 0 for a candidate the grid
  * does not take) may each be NULL.  Per-q-point grids have one shape: best_ppt = 0. */
 int hgx_ff_tune(hgx_ctx ctx, hgx_qgrid g, const double* shape_def, int ntri,
                 const double* rot9, int ff_type, int reps, int* best_ppt, double* best_ms,

@@ -34,11 +34,13 @@ __device__ __forceinline__ void signed_digits(const uint32_t (&w)[4], uint32_t (
 // in the combined sum's.
 __device__ __forceinline__ uint32_t offset_units(long long sum) { return (uint32_t)(sum >> 10); }
 __device__ __forceinline__ float offset_rest(long long sum) { return (float)((int)(sum & 1023) << 6) * S36; }
-// A column's combined sum less that offset, from its four accumulators s_i (weights 2^24, 2^16, 2^8, 1 units).
-__device__ __forceinline__ float combined_sum(uint32_t s0, uint32_t s1, uint32_t s2, uint32_t s3, uint32_t units,
-                                              float rest) {
-  const float lo = fmaf((float)(int)s2, 256.f * S36, fmaf((float)(int)s3, S36, -rest));
-  return fmaf((float)(int)(s0 * 256u + s1 - units), 65536.f * S36, lo);
+// A column's combined sum less that offset, from its four accumulators s_i (weights 2^24, 2^16, 2^8, 1 units):
+// the low two's part, and the whole.
+__device__ __forceinline__ float low_sum(uint32_t s2, uint32_t s3, float rest) {
+  return fmaf((float)(int)s2, 256.f * S36, fmaf((float)(int)s3, S36, -rest));
+}
+__device__ __forceinline__ float combined_sum(uint32_t s0, uint32_t s1, uint32_t units, float low) {
+  return fmaf((float)(int)(s0 * 256u + s1 - units), 65536.f * S36, low);
 }
 
 // The digits of the phasors e^{i q.d} of this thread's q with 16 offsets d (or of its offset with

@@ -29,7 +29,7 @@
 //
 // What bounds it: the digits.  Per (pixel, triangle) two SFU operations and about 14 issued
 // instructions (PRMT 3.6, FFMA2 1.5, LOP3 1.3, FMUL 1.2): SFU 76%, issue 66%; the products take
-// 150 of the 690 cycles of a chunk.  2048 x 2048 x 50,000: 129 ms with 20 digit warps of 80
+// 150 of the 690 cycles of a chunk.  2048 x 2048 x 50,000: 128 ms with 20 digit warps of 80
 // registers (with three digits of the row factors 126, and then 24 warps of 72: 129, 16 of 96: 147, three
 // warpgroups of 168 registers, each with its own pixels: 148), against 190 ms for the FP32 row kernel, whose 16
 // FFMA per (pixel, triangle) of accumulation these products replace.  Taking a quarter of the sines off the SFU by polynomials on the
@@ -242,14 +242,17 @@ __device__ __forceinline__ void add_tile_sums(const MmaArgs& a, uint32_t d_tm, i
     float f[2][6];  // sums with cos, with sin: (n~x, n~y, n~z) Re Z, then Im Z
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      uint32_t d[32];
+      uint32_t d[16];  // two slices at a time
 #pragma unroll
-      for (int i = 0; i < 4; ++i) tmem_ld8(d_tm + k * S::D_COLS + i * S::NP + 6 * u, d + 8 * i);
-      tmem_wait_ld<32>(d);
+      for (int i = 0; i < 2; ++i) tmem_ld8(d_tm + k * S::D_COLS + (2 + i) * S::NP + 6 * u, d + 8 * i);
+      tmem_wait_ld<16>(d);
 #pragma unroll
-      for (int j = 0; j < 6; ++j)
-        f[k][j] = combined_sum(d[j], d[8 + j], d[16 + j], d[24 + j], rec[6 * u + j],
-                               __uint_as_float(rec[7 * U + 6 * u + j]));
+      for (int j = 0; j < 6; ++j) f[k][j] = low_sum(d[j], d[8 + j], __uint_as_float(rec[7 * U + 6 * u + j]));
+#pragma unroll
+      for (int i = 0; i < 2; ++i) tmem_ld8(d_tm + k * S::D_COLS + i * S::NP + 6 * u, d + 8 * i);
+      tmem_wait_ld<16>(d);
+#pragma unroll
+      for (int j = 0; j < 6; ++j) f[k][j] = combined_sum(d[j], d[8 + j], rec[6 * u + j], f[k][j]);
     }
     const float *fc = f[0], *fs = f[1];
     const double2 q = a.rowqz[(long)row * NK + (PAIRED ? 2 * u : u)];

@@ -210,7 +210,7 @@ __device__ __forceinline__ void bwm_add(uint32_t d_tm, const uint32_t* rec, doub
       for (int j = 0; j < 8; ++j) {
         const int c = 12 * pr + 8 * h + j;
         if (8 * h + j < 12) {
-          f[8 * h + j] = combined_sum(d[j], d[8 + j], d[16 + j], d[24 + j], rec[c], __uint_as_float(rec[48 + c])) *
+          f[8 * h + j] = combined_sum(d[j], d[8 + j], rec[c], low_sum(d[16 + j], d[24 + j], __uint_as_float(rec[48 + c]))) *
                          __uint_as_float(rec[24 + c]);
         }
       }

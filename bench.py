@@ -36,21 +36,21 @@ QMIN_Y, QMIN_Z, QMAX_Y, QMAX_Z = -2.0, 0.0, 2.0, 3.0
 ENERGY_KEV, ALPHA_I_DEG = 10.0, 0.20
 PI_REF = 3.141592653589793
 # The row kernel per (pixel, triangle) with the 4 paired real DWBA blocks: 2 SFU operations
-# (sin, cos of the in-plane phase) and, on the tensor cores, 192 int8 products (3 digits of each x
-# 96 columns of row-factor digits).  The factorised sum written with FP32 operations (FMA = 2): phase 3, q_par.n~ 3, U 2,
+# (sin, cos of the in-plane phase) and, on the tensor cores, 288 int8 products (the 3 digits of each x
+# 64, 48 and 32 columns of row-factor digits).  The factorised sum written with FP32 operations (FMA = 2): phase 3, q_par.n~ 3, U 2,
 # 16 accumulating FMA 32 -> 40 FLOP.
 FLOP_PER_PIXEL_TRI = 40.0
 SFU_PER_PIXEL_TRI = 2.0
-INT8_OPS_PER_PIXEL_TRI = 384.0
-# DRAM bytes per step: the row factors' digits (2048 rows x 98 tiles x 24,640 bytes) written and
-# read once, the q-grid and the output.  At 512 x 512 x 20,000 ncu counts 444 MB written and 510 MB
-# read for 504 MB of digits.
-TRAFFIC_BYTES_PER_LAUNCH = 2 * 4.95e9 + 201.0e6
-TRAFFIC_SOURCE = "row-factor digits 2 x 4.95 GB (by layout; ncu at 512x512 agrees), q-grid and output"
+INT8_OPS_PER_PIXEL_TRI = 576.0
+# DRAM bytes per step: the row factors' digits (2048 rows x 98 tiles x 32,880 bytes) written and
+# read once, the q-grid and the output.  At 512 x 512 x 20,000 ncu counts 612 MB written and 680 MB
+# read for 673 MB of digits.
+TRAFFIC_BYTES_PER_LAUNCH = 2 * 6.60e9 + 201.0e6
+TRAFFIC_SOURCE = "row-factor digits 2 x 6.60 GB (by layout; ncu at 512x512 agrees), q-grid and output"
 # the library's kernels per form-factor step (bounding box 2, Morton keys, tiles, and for each of
-# five slabs of row factors their kernel and the row kernel);
+# seven slabs of row factors their kernel and the row kernel);
 # CUB's radix sort of the keys adds 6 launches per step
-HGX_LAUNCHES_PER_STEP = 14
+HGX_LAUNCHES_PER_STEP = 18
 CUB_LAUNCHES_PER_STEP = 6
 
 
@@ -59,23 +59,23 @@ CUB_LAUNCHES_PER_STEP = 6
 # each from an ncu capture of its kernel on the workload below:
 #   (the mesh vertex gradient is held against the SFU: 2 operations per pass and (pixel, triangle))
 #   ff_exact_kernel          611 FP64 per (q-point, triangle)
-#   grain_dwba_real_kernel<double>  363 FP64 per (pixel, grain), hcp cylinders (HIG_ENSEMBLE)
-#   grain_dwba_real_kernel<float>   147 FP32 + 68 FP64 per (pixel, grain), the same description
+#   grain_dwba_real_kernel<double>  366 FP64 per (pixel, grain), hcp cylinders (HIG_ENSEMBLE)
+#   grain_dwba_real_kernel<float>   176 FP32 + 70 FP64 per (pixel, grain), the same description
 #   cyl_pixels_f32c_kernel   200 FP32 + 52 FP64 per ROI pixel (FP32x2 counted as two)
 #   cyl_pixels_kernel<double>  1418 FP64 per ROI pixel (the same batch)
-#   grain_dwba_real_kernel<float>   978 FP32 + 307 FP64 and 118 XU-pipe operations per pixel (config 1)
-#   grain_dwba_real_kernel<double>  1414 FP64 per pixel (config 1)
+#   grain_dwba_real_kernel<float>   970 FP32 + 309 FP64 and 120 XU-pipe operations per pixel (config 1)
+#   grain_dwba_real_kernel<double>  1437 FP64 per pixel (config 1)
 CYL_F32C_FP32_FLOP_PER_PIXEL = 200.0
 CYL_F32C_FP64_FLOP_PER_PIXEL = 52.0
 CYL_F64_FLOP_PER_PIXEL = 1418.0
-CFG1_F32C_FP32_FLOP_PER_PIXEL = 978.0
-CFG1_F32C_FP64_FLOP_PER_PIXEL = 307.0
-CFG1_F32C_XU_PER_PIXEL = 118.0
-CFG1_F64_FLOP_PER_PIXEL = 1414.0
+CFG1_F32C_FP32_FLOP_PER_PIXEL = 970.0
+CFG1_F32C_FP64_FLOP_PER_PIXEL = 309.0
+CFG1_F32C_XU_PER_PIXEL = 120.0
+CFG1_F64_FLOP_PER_PIXEL = 1437.0
 EXACT_FP64_FLOP_PER_EVAL = 611.0
-GRAIN_FP64_FLOP_PER_PIXEL_GRAIN = 363.0
-GRAIN_F32C_FP32_FLOP_PER_PIXEL_GRAIN = 147.0
-GRAIN_F32C_FP64_FLOP_PER_PIXEL_GRAIN = 68.0
+GRAIN_FP64_FLOP_PER_PIXEL_GRAIN = 366.0
+GRAIN_F32C_FP32_FLOP_PER_PIXEL_GRAIN = 176.0
+GRAIN_F32C_FP64_FLOP_PER_PIXEL_GRAIN = 70.0
 
 
 def roofline_of(bound, flop_per_unit, units, seconds, peak, unit, source):
@@ -943,7 +943,7 @@ def main():
         npx1 = float(cfg1["pixels"])
         t32, t64 = cfg1["f32c"]["ms"] * 1e-3, cfg1["f64"]["ms"] * 1e-3
         r32 = roofline_of("fp32", CFG1_F32C_FP32_FLOP_PER_PIXEL, npx1, t32, peak_fp32, "pixel",
-                          "ncu executed FP32 FLOP of grain_dwba_real_kernel (plus 307 FP64 per pixel); "
+                          "ncu executed FP32 FLOP of grain_dwba_real_kernel (plus 309 FP64 per pixel); "
                           "the time is the whole simulation (set-up, Fresnel coefficients, grain kernel, sums)")
         xu = CFG1_F32C_XU_PER_PIXEL * npx1 / t32 / 1e9
         r32["sfu"] = {"ops_per_unit": CFG1_F32C_XU_PER_PIXEL, "achieved_gops": xu, "peak_gops": peak_sfu,

@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(128) ff_analytic_kernel(const AnaArgs* __restr
 // Grids with real qz blocks (ana_sf_real.cuh), T = double or float (FP32C: FP64 phases, FP32
 // transcendentals and sums); SHAPE: cylinder, sphere or box.  One thread per pixel makes the four
 // blocks, the in-plane sums once where the rotation keeps qz out of them.  Bound by the FP64 pipe;
-// at 640 x 481 a cylinder of 11 + 11 samples: 0.042 ms, 0.44 in the complex form of
+// at 640 x 481 a cylinder of 11 + 11 samples: 0.040 ms, 0.44 in the complex form of
 // ff_analytic_kernel; a sphere of 5 samples: 0.039, 0.149.
 template <typename T, int SHAPE, typename OUT>
 __global__ void __launch_bounds__(128) ff_analytic_real_kernel(const AnaArgs* __restrict__ ap) {

@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(128, (SHAPE == SH_PYRAMID || SHAPE == 0) ? 3 :
 //
 // Bound by the FP64 pipe (T = double: 230 FP64 operations per (pixel, grain) with a c axis, where
 // grain_dwba_kernel's complex powers, logarithms and exponentials take 6,400) or by issue (float).
-// 600 x 300 pixels x 625 grains, 100 x 10 x 2 cells: FP64 2.16 ms (63.5 on grain_dwba_kernel), FP32C
+// 600 x 300 pixels x 625 grains, 100 x 10 x 2 cells: FP64 2.18 ms (63.5 on grain_dwba_kernel), FP32C
 // 1.3 ms (10.0 on four threads per pixel); four CTAs of 128 registers per SM (3: 3.2 ms, 6: 2.6 at
 // an earlier step of 2.5).  Grains of a launch are split over grid z where a small image leaves
 // SMs idle; grain_sum_kernel adds the splits' sums in order.

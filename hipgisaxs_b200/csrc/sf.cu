@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(128) sf_lattice_kernel(SfArgs a) {
 // Grids with real qz blocks (ana_sf_real.cuh), T = double or float (FP32C: FP64 phase reduction,
 // FP32 sines).  One thread per pixel makes the four blocks: the a- and b-axis factors once where
 // the rotation keeps qz out of them, angles as q . (rotated vector) in turns.  Bound by the FP64
-// pipe; 640 x 481 pixels: 0.011 ms, where the complex powers of sf_lattice_kernel take 0.125.
+// pipe; 640 x 481 pixels: 0.012 ms, where the complex powers of sf_lattice_kernel take 0.125.
 struct SfRealArgs {
   double a[3], b[3], c[3], d[3], b0, rep[3];
   const double* qx;

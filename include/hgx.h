@@ -103,7 +103,7 @@ int hgx_ff_triangles_q(hgx_ctx ctx, hgx_qgrid g, const double* shape_def, int nt
  * pixels_per_thread 1, 2 or 4 selects the scalar kernel with that many pixels per thread;
  * -2, -4 or -8 the packed FP32x2 kernel (paired real grids only); 0 = automatic: the shape that
  * hgx_ff_tune stored in the grid if any, else on row grids nearly always the tensor-core kernel (which
- * has one shape and keeps up to 1 GiB of row factors in the context), else scalar with 4, fewer when the
+ * has one shape and keeps up to 1 GiB of row factors, or one row's, in the context), else scalar with 4, fewer when the
  * grid is too small to fill the GPU. */
 int hgx_ff_triangles_q_ex(hgx_ctx ctx, hgx_qgrid g, const double* shape_def, int ntri,
                           const double* rot9, int precision, void* ff, int ff_type,
@@ -400,7 +400,7 @@ int hgx_mesh_to_shape_def(hgx_ctx ctx, int nv, const double* verts, int nf, cons
  * coefficients (nrow x 4); chi^2 = sum mask (scale I - counts)^2 / max(counts, 1).
  * Outputs: chi2 (host double), grad_verts (nv x 3, may be NULL), intensity (N, may be
  * NULL).  The grid must be a DWBA grid with real qz constant along rows.  On grids wider than
- * 128 columns the context keeps up to 1 GiB of seed digits (the same block as the form factor's row
+ * 128 columns the context keeps up to 1 GiB of seed digits, or one row's (the same block as the form factor's row
  * factors) and, on any, partial sums of 48 bytes per face and row range (64 MiB or one range). */
 int hgx_mesh_chi2_grad(hgx_ctx ctx, hgx_qgrid g, int nv, const double* verts, int nf,
                        const int* faces, const double* rot9, const double* rowfc,

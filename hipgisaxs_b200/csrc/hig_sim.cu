@@ -565,38 +565,43 @@ static void launch_grain_real(GrainKernel k, int shape, bool f32c, dim3 grid, cu
 #undef HGX_QUAD_LAUNCH
 }
 
-// Which kernel a structure on real qz takes.  npix: pixels of a launch; samples: the largest number of samples of
-// a dimension; flat: no rotation takes qz into the rotated in-plane q and no a vector has a z component.
-// FP32C: a thread per pixel shares the in-plane sums among the blocks of flat grains and keeps the form factors
-// of successive ones; where there is nothing to share (tilted grains, boxes of several samples, one grain of
-// spheres) or too few pixels the quad kernel is the faster one.  Times in ms, pixel / quad kernel: 257 x 200 x
-// 9 tilted grains of boxes of 11 samples 0.275 / 0.193, of cylinders 0.188 / 0.148; 100 x 80 x 2 tilted boxes 0.073 /
-// 0.036; 40 x 28, one flat grain of cylinders 0.031 / 0.025; on the other side 600 x 300 x 60 flat grains of
-// cylinders 0.102 / 0.84, of boxes of one sample 0.59 / 0.91, tilted ones of spheres 0.73 / 0.88.
+// Which kernel a structure on real qz takes, by what its grains share.
+struct GrainTraits {
+  int samples = 1;     // largest number of samples of a dimension
+  bool tilted = false; // some rotation takes qz into an element's in-plane q: the blocks share no sums
+  bool kept = false;   // successive grains have the same form factors (grain_dwba_real_kernel's keep)
+  int nelem = 0;
+  GrainTraits(int shape, const std::vector<AnaShape>& shapes, const std::vector<FusedElem>& elems,
+              const std::vector<double>& er) {
+    for (const AnaShape& s : shapes)
+      for (const Dist& d : s.d) samples = std::max(samples, d.n);
+    for (size_t i = 0; i < er.size(); i += 9) tilted = tilted || er[i + 2] != 0.0 || er[i + 5] != 0.0;
+    kept = shape != SH_BOX && !tilted;
+    for (const FusedElem& e : elems) kept = kept && e.loc[0] == 0.0 && e.loc[1] == 0.0;
+    nelem = (int)elems.size();
+  }
+};
+// FP32C: a thread per pixel shares the in-plane sums among the blocks and keeps the form factors of successive
+// grains; the quad kernel is the faster one where there is less to share than to gain from its occupancy (tilted
+// grains, many samples) or too few pixels and grains for one thread and a split each (npix: pixels of a launch).
+// Times in ms, pixel / quad kernel: 257 x 200 x 9 tilted grains of boxes of 11 samples 0.275 / 0.193, of cylinders
+// 0.188 / 0.148; 600 x 300 x 9 flat boxes of 11 samples 0.405 / 0.333; 600 x 300 x 16 pairs of spheres of 11
+// samples off the axis 1.31 / 1.08, threes of 4 samples 0.82 / 0.74; 40 x 28 x 4 pairs of cylinders 0.093 / 0.048;
+// on the other side 600 x 300 x 60 flat grains of cylinders 0.102 / 0.84, of boxes of one sample 0.59 / 0.91, of
+// four 1.07 / 1.57, tilted spheres 0.73 / 0.88, 120 x 90 x 60 boxes of four samples 0.098 / 0.141.
 // FP64: a few tilted grains of cylinders on few pixels go to the complex kernel's four threads per pixel (40 x 28,
 // 11 samples: 0.061 / 0.049).
-static GrainKernel grain_real_plan(int shape, bool f32c, int samples, bool flat, long npix, int ngrains) {
-  const bool few = npix < 40000, single = samples <= 2;
-  if (!f32c) return shape == SH_CYLINDER && !flat && !single && npix < 6000 && ngrains <= 4 ? GRAIN_COMPLEX : GRAIN_PIXEL;
-  if (!flat) return shape == SH_BOX || !single || (few && ngrains < 32) ? GRAIN_QUAD : GRAIN_PIXEL;
-  if (shape == SH_BOX) return !single || (few && ngrains <= 2) ? GRAIN_QUAD : GRAIN_PIXEL;
-  return (few && ngrains <= 2) || (shape == SH_SPHERE && !single && ngrains == 1) ? GRAIN_QUAD : GRAIN_PIXEL;
-}
-
-static int grain_samples(const std::vector<AnaShape>& shapes) {
-  int n = 1;
-  for (const AnaShape& s : shapes)
-    for (const Dist& d : s.d) n = std::max(n, d.n);
-  return n;
-}
-static bool grains_flat(const std::vector<double>& gt, const std::vector<double>& er, const std::vector<ScaleEntry>& plan) {
-  for (size_t i = 0; i < gt.size(); i += 12)
-    if (gt[i + 2] != 0.0 || gt[i + 5] != 0.0) return false;
-  for (size_t i = 0; i < er.size(); i += 9)
-    if (er[i + 2] != 0.0 || er[i + 5] != 0.0) return false;
-  for (const ScaleEntry& e : plan)
-    if (e.la[2] != 0.0) return false;
-  return true;
+static GrainKernel grain_real_plan(int shape, bool f32c, const GrainTraits& t, long npix, int ngrains) {
+  const bool few = npix < 40000;
+  if (!f32c)
+    return shape == SH_CYLINDER && t.tilted && t.samples > 2 && npix < 6000 && ngrains <= 4 ? GRAIN_COMPLEX : GRAIN_PIXEL;
+  if (few && ngrains < (t.kept ? 3 : t.tilted ? 32 : 8)) return GRAIN_QUAD;
+  bool quad;
+  if (t.tilted) quad = shape == SH_BOX || t.samples > 2;
+  else if (shape == SH_CYLINDER) quad = !t.kept && t.samples > 7 && (ngrains > 1 || t.nelem > 1);
+  else if (shape == SH_SPHERE) quad = (!t.kept || ngrains == 1) && t.samples > 3;
+  else quad = t.samples > 7;
+  return quad ? GRAIN_QUAD : GRAIN_PIXEL;
 }
 
 // The tangent of the fused grain loop (FP64, real qz): for one direction of the fit
@@ -1175,8 +1180,7 @@ static int fused_structure(hgx_ctx c, hgx_qgrid g, HigWork& w, const hig::Struct
     if (shapes[e].shape != one) one = 0;
   // grids with real qz blocks (paired rows) and one shape with a real-qz body
   const bool real = g->mode == 1 && grain_real_shape(one), f32c = precision == HGX_F32C;
-  const GrainKernel plan_k = real ? grain_real_plan(one, f32c, grain_samples(shapes), grains_flat(gt, er, plan), a.n, ngr)
-                                  : GRAIN_COMPLEX;
+  const GrainKernel plan_k = real ? grain_real_plan(one, f32c, GrainTraits(one, shapes, elems, er), a.n, ngr) : GRAIN_COMPLEX;
   if (plan_k != GRAIN_COMPLEX) {
     const unsigned ctas = grain_real_ctas(plan_k, a.n);
     // four CTAs of 128 threads run per SM (nine of the quad kernel); grains are split where the pixels do not fill them
@@ -2141,9 +2145,13 @@ int hgx_hig_population_eval(hgx_hig_pop p, const double* X, int nx, double* dist
     const PopStruct& ps = p->st[k];
     GrainKernel gk = GRAIN_COMPLEX;
     if (ps.real) {
-      bool flat = true;
-      for (const auto& T : all) flat = flat && grains_flat(T[k].f.gt, T[k].f.er, T[k].plan);
-      gk = grain_real_plan(ps.shape, ps.f32c, grain_samples(all[0][k].f.shapes), flat, p->n * p->npop, ps.ngr);
+      GrainTraits t(ps.shape, all[0][k].f.shapes, all[0][k].f.elems, all[0][k].f.er);
+      for (const auto& T : all) {
+        const GrainTraits c(ps.shape, T[k].f.shapes, T[k].f.elems, T[k].f.er);
+        t.tilted = t.tilted || c.tilted;
+        t.kept = t.kept && c.kept;
+      }
+      gk = grain_real_plan(ps.shape, ps.f32c, t, p->n * p->npop, ps.ngr);
     }
     for (int g0 = 0; g0 < ps.ngr; g0 += chunk)
       v.push_back(gk != GRAIN_COMPLEX ? (int)gk : -1 - (int)pop_paired(all, k, g0, std::min(ps.ngr, g0 + chunk)));
